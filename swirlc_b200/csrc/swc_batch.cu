@@ -432,11 +432,12 @@ extern "C" int swc_batch_step(const SwcScheme* sc, int32_t order,
     if (rc) return rc;
   }
   // Tiles: 16x16 unless the member asks for 8x32 (which suits members at
-  // most 8 cells wide in y, and whose shared-memory layout does not fit for
-  // f64 WENO5). The 16x16 instance reproduces swc_rk_step bit for bit; the
+  // most 8 cells wide in y, and is not offered for f64 WENO5, whose layout
+  // fills the whole of shared memory). The 16x16 instance reproduces swc_rk_step bit for bit; the
   // 8x32 instance of the same arithmetic is scheduled differently by the
   // compiler and can differ from it in the last bit.
-  const bool narrow_ok = batch_smem(sc, 2) <= kSmemLimit;
+  const bool narrow_ok = (sc->dtype == SWC_F32 || sc->interp != SWC_WENO5) &&
+                         batch_smem(sc, 2) <= kSmemLimit;
   std::vector<Plan> plans(nmembers);
   for (int i = 0; i < nmembers; ++i) {
     plans[i].m = &members[i];

@@ -238,20 +238,18 @@ __global__ void riemann_kernel(const PointArgs a) {
     T pdl = a.pdl ? static_cast<const T*>(a.pdl)[i] : l.p;
     T pdr = a.pdr ? static_cast<const T*>(a.pdr)[i] : r.p;
     T pe = a.pe ? static_cast<const T*>(a.pe)[i] : T(0);
-    T f[5];
-    if constexpr (RM == 0) hll_flux<T, D>(l, r, pdl, pdr, pe, f);
-    else hllc_flux<T, D>(l, r, pdl, pdr, pe, f);
+    T f[5], phl[3], phr[3], fs[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      phl[k] = k < a.ns ? static_cast<const T*>(a.ql[7 + k])[i] : T(0);
+      phr[k] = k < a.ns ? static_cast<const T*>(a.qr[7 + k])[i] : T(0);
+    }
+    face_flux<RM, T, D, 3>(l, r, pdl, pdr, pe, phl, phr, f, fs);
 #pragma unroll
     for (int k = 0; k < 5; ++k) static_cast<T*>(a.out[k])[i] = f[k];
-    if (a.ns > 0) {
-      T phl[3], phr[3], fs[3];
-      for (int k = 0; k < a.ns; ++k) {
-        phl[k] = static_cast<const T*>(a.ql[7 + k])[i];
-        phr[k] = static_cast<const T*>(a.qr[7 + k])[i];
-      }
-      scalar_fluxes<RM, T, D>(l, r, pdl, pdr, pe, a.ns, phl, phr, fs);
-      for (int k = 0; k < a.ns; ++k) static_cast<T*>(a.out[5 + k])[i] = fs[k];
-    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+      if (k < a.ns) static_cast<T*>(a.out[5 + k])[i] = fs[k];
   }
 }
 
@@ -264,10 +262,12 @@ __global__ void speeds_kernel(const PointArgs a) {
     load_prim<T, D>(a.qr, i, r);
     T pe = a.pe ? static_cast<const T*>(a.pe)[i] : T(0);
     T s_l, s_r;
-    hll_speeds<T, D>(l, r, pe, s_l, s_r);
+    hll_speeds<T, D>(l, r, l.p, r.p, One<T>::rcp(l.r), One<T>::rcp(r.r), pe,
+                     s_l, s_r);
     static_cast<T*>(a.sl)[i] = s_l;
     static_cast<T*>(a.sr)[i] = s_r;
-    if (a.sm) static_cast<T*>(a.sm)[i] = hllc_contact<T, D>(l, r, s_l, s_r);
+    if (a.sm)
+      static_cast<T*>(a.sm)[i] = hllc_contact<T, D>(l, r, l.p, r.p, s_l, s_r);
   }
 }
 
@@ -335,11 +335,10 @@ __global__ void viscous_terms_kernel(const ViscArgs a) {
   const T* qv[5];
 #pragma unroll
   for (int v = 0; v < 5; ++v) qv[v] = static_cast<const T*>(a.q[v]);
-  const T h[3] = {T(a.h[0]), T(a.h[1]), T(a.h[2])};
-  const T rh[3] = {rcp_(h[0]), rcp_(h[1]), rcp_(h[2])};
-  const T r2h[3] = {rcp_(T(2) * h[0]), rcp_(T(2) * h[1]), rcp_(T(2) * h[2])};
+  using O = One<T>;
+  const T rh[3] = {rcp_(T(a.h[0])), rcp_(T(a.h[1])), rcp_(T(a.h[2]))};
   const T nu = a.what == SWC_VISC_STRAIN ? T(0.5) : T(a.nu);
-  const T inv_pr = T(1.0 / a.pr);
+  const T kq = heat_coefficient<T>(a.pr);
   const bool zero_vel = a.what == SWC_VISC_HEAT;
   const bool cell_rho_p = a.what == SWC_VISC_FLUX || a.what == SWC_VISC_HEAT;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n;
@@ -362,23 +361,25 @@ __global__ void viscous_terms_kernel(const ViscArgs a) {
       if (ok) {
         const long long ob = o, oa = o - st[dn];
         const int vel[3] = {1 + dn, 1 + t1, 1 + t2};
-        T ua[3], ub[3], ga[3][3] = {}, gb[3][3] = {};
+        T ua[3], ub[3];
+        T g11 = T(0), g10 = T(0), g22 = T(0), g20 = T(0);
         if (!zero_vel) {
 #pragma unroll
           for (int c = 0; c < 3; ++c) {
             ua[c] = qv[vel[c]][oa];
             ub[c] = qv[vel[c]][ob];
           }
-          const T i2t1 = T(2) * h[t1], i2t2 = T(2) * h[t2];
-          const long long s1 = st[t1], s2 = st[t2];
-          ga[1][1] = divk(qv[vel[1]][oa + s1] - qv[vel[1]][oa - s1], i2t1, r2h[t1]);
-          gb[1][1] = divk(qv[vel[1]][ob + s1] - qv[vel[1]][ob - s1], i2t1, r2h[t1]);
-          ga[1][0] = divk(qv[vel[0]][oa + s1] - qv[vel[0]][oa - s1], i2t1, r2h[t1]);
-          gb[1][0] = divk(qv[vel[0]][ob + s1] - qv[vel[0]][ob - s1], i2t1, r2h[t1]);
-          ga[2][2] = divk(qv[vel[2]][oa + s2] - qv[vel[2]][oa - s2], i2t2, r2h[t2]);
-          gb[2][2] = divk(qv[vel[2]][ob + s2] - qv[vel[2]][ob - s2], i2t2, r2h[t2]);
-          ga[2][0] = divk(qv[vel[0]][oa + s2] - qv[vel[0]][oa - s2], i2t2, r2h[t2]);
-          gb[2][0] = divk(qv[vel[0]][ob + s2] - qv[vel[0]][ob - s2], i2t2, r2h[t2]);
+          // Central differences along an axis of stride sv, averaged over
+          // the two cells.
+          auto diff = [&](const T* q, long long sv, T rhv) -> T {
+            return O::mul(O::add(O::sub(q[oa + sv], q[oa - sv]),
+                                 O::sub(q[ob + sv], q[ob - sv])),
+                          O::mul(T(0.25), rhv));
+          };
+          g11 = diff(qv[vel[1]], st[t1], rh[t1]);
+          g10 = diff(qv[vel[0]], st[t1], rh[t1]);
+          g22 = diff(qv[vel[2]], st[t2], rh[t2]);
+          g20 = diff(qv[vel[0]], st[t2], rh[t2]);
         } else {
 #pragma unroll
           for (int c = 0; c < 3; ++c) ua[c] = ub[c] = T(0);
@@ -394,14 +395,14 @@ __global__ void viscous_terms_kernel(const ViscArgs a) {
         }
         const T pa = cell_rho_p ? qv[4][oa] : T(1);
         const T pb = cell_rho_p ? qv[4][ob] : T(1);
-        T f[5] = {T(0), T(0), T(0), T(0), T(0)};
-        viscous_flux<T, 0>(ra, rb, ua, ub, pa, pb, ga, gb, h[dn], rh[dn], nu,
-                           inv_pr, f);
+        T f[4];
+        viscous_flux<T>(ra, rb, ua, ub, pa, pb, g11, g10, g22, g20, rh[dn], nu,
+                        kq, f);
         // Back to (x, y, z) momentum order.
-        fo[1] = dn == 0 ? f[1] : f[2];
-        fo[2] = dn == 1 ? f[1] : (dn == 0 ? f[2] : f[3]);
-        fo[3] = dn == 2 ? f[1] : f[3];
-        fo[4] = f[4];
+        fo[1] = dn == 0 ? f[0] : f[1];
+        fo[2] = dn == 1 ? f[0] : (dn == 0 ? f[1] : f[2]);
+        fo[3] = dn == 2 ? f[0] : f[2];
+        fo[4] = f[3];
       }
       if (a.what == SWC_VISC_FLUX) {
 #pragma unroll

@@ -11,14 +11,16 @@
 // of RING planes of primitives (with an in-plane halo HR) lives in shared
 // memory; each step computes every y- and x-face of the centre plane into
 // shared memory and the z-face above each column in registers (the face
-// below is carried from the previous step), converts the next plane into a
-// ring slot those faces do not read, and after the step's one barrier forms
+// below is carried from the previous step), converts the next plane, which
+// arrived in its ring slot meanwhile, and after the step's one barrier forms
 // the divergence and the stage update of the centre plane. Each face flux is
 // computed exactly once per CTA. x and y faces reconstruct both face states
 // from the face's stencil; z faces take them from cell-centred
 // reconstructions of the column's cells, one per cell, whose upper-face
 // value is carried up the column. The primitives are reconstructed two at a
-// time (f32x2 lanes), all with explicitly rounded operations.
+// time (f32x2 lanes) and stored two at a time: one 8-byte shared-memory load
+// (16 in double precision) brings both lanes of a stencil cell into a
+// register pair. Everything up to the stage update is explicitly rounded.
 #pragma once
 
 #include <type_traits>
@@ -89,29 +91,45 @@ struct Geom {
 };
 
 // Shared-memory layout. NS transported scalars and (HELP) the p_dyn helper
-// add reconstructed variables to the 7 primitives rho, u, v, w, e, p, h.
+// add reconstructed variables to the 7 primitives. A ring slot holds the
+// variables (rho, e), (u, v), (w, p), (h, x0), (x1, x2) .. as arrays of pairs
+// and, when their number is odd, the last one alone; x0, x1 .. are the
+// scalars, then p_dyn. An incoming plane is copied straight into the pair
+// positions of its slot (rho_u where u goes, p_ref where p_dyn goes) and
+// converted in place, each cell by the thread that copied it.
 template <typename T, int SCHEME, bool VISC, int TY, int TX, int NS = 0,
           bool HELP = false>
 struct Layout {
   using G = Geom<SCHEME, VISC>;
-  static constexpr int NV = 7 + NS + (HELP ? 1 : 0);   // ring variables
-  static constexpr int NCS = 5 + NS + (HELP ? 1 : 0);  // staged fields
-  static constexpr int NF = 5 + NS;                     // flux components
+  static constexpr int NV = 7 + NS + (HELP ? 1 : 0);  // ring variables
+  static constexpr int NP = NV / 2;                   // pairs
+  static constexpr int NF = 5 + NS;                   // flux components
   static constexpr int PW = TY + 2 * G::HR;
   static constexpr int PH = TX + 2 * G::HR;
   static constexpr int PS = PW * PH;
   static constexpr int NT = TX * TY;
   static constexpr int PER = (PS + NT - 1) / NT;  // plane cells per thread
-  static constexpr int RING_ELEMS = G::RING * NV * PS;
-  static constexpr int STAGE_ELEMS = NCS * PS;
+  static constexpr int SLOT = (NV * PS + 3) / 4 * 4;  // 16-byte multiple
+  static constexpr int RING_ELEMS = G::RING * SLOT;
   // x- and y-face fluxes, two buffers each (planes alternate), so that
   // threads may start the next plane's faces while others still form the
   // update of this one. The z-face flux stays in the registers of the
-  // thread that computes and uses it.
-  static constexpr int FY_ELEMS = NF * TX * (TY + 1);
-  static constexpr int FX_ELEMS = NF * (TX + 1) * TY;
+  // thread that computes and uses it. Components as (rho, rho_e),
+  // (rho_u, rho_v), (rho_w, scalar 0) .. pairs and the last one alone.
+  static constexpr int NFP = NF / 2;
+  static constexpr int NY = TX * (TY + 1), NX = (TX + 1) * TY;
+  static constexpr int FY_ELEMS = (NF * NY + 3) / 4 * 4;
+  static constexpr int FX_ELEMS = (NF * NX + 3) / 4 * 4;
   static constexpr size_t SMEM =
-      sizeof(T) * (size_t)(RING_ELEMS + STAGE_ELEMS + 2 * (FY_ELEMS + FX_ELEMS));
+      sizeof(T) * (size_t)(RING_ELEMS + 2 * (FY_ELEMS + FX_ELEMS));
+  // Offset in a ring slot of variable q (in the order rho, e, u, v, w, p, h,
+  // x0 ..) of plane cell 0, and the step from one cell to the next.
+  __host__ __device__ static constexpr int var_off(int q) {
+    return q / 2 < NP ? (q / 2) * 2 * PS + (q & 1) : 2 * NP * PS;
+  }
+  __host__ __device__ static constexpr int var_step(int q) {
+    return q / 2 < NP ? 2 : 1;
+  }
 };
 
 // 4- or 8-byte asynchronous global->shared copy (LDGSTS), cached in L1 so
@@ -149,27 +167,33 @@ __device__ __forceinline__ void stage_body(const StageArgs& a,
                                            const int x0, const int zb) {
   using G = Geom<SCHEME, VISC>;
   using L = Layout<T, SCHEME, VISC, TY, TX, NS, HELP>;
-  constexpr int NV = L::NV, NCS = L::NCS, NF = L::NF;
+  using O1 = One<T>;
+  using O2 = Two<T>;
+  using V2 = typename O2::V;
+  constexpr int NV = L::NV, NP = L::NP, NF = L::NF, NFP = L::NFP;
   constexpr int LO = G::LO, NW = G::NW, HR = G::HR, ZLO = G::ZLO,
                 ZHI = G::ZHI, RING = G::RING, SPARE = G::SPARE, CL = G::CL,
-                CW = G::CW, NOFF = G::NOFF;
-  constexpr int PW = L::PW, PH = L::PH, PS = L::PS, NT = L::NT, PER = L::PER;
+                CW = G::CW;
+  constexpr int PW = L::PW, PS = L::PS, NT = L::NT, PER = L::PER;
+  constexpr int SLOT = L::SLOT;
 
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* ring = reinterpret_cast<T*>(smem_raw);
-  T* stg = ring + L::RING_ELEMS;    // [NCS][PS] conserved plane in flight
-  T* fy0 = stg + L::STAGE_ELEMS;    // [2][NF][TX][TY+1]
-  T* fx0 = fy0 + 2 * L::FY_ELEMS;   // [2][NF][TX+1][TY]
+  T* const ring = reinterpret_cast<T*>(smem_raw);
+  T* const fy0 = ring + L::RING_ELEMS;
+  T* const fx0 = fy0 + 2 * L::FY_ELEMS;
 
   const int tid = threadIdx.x;
-  // Cell of this thread. For TY = 16 a warp covers rows w and w + TX/2, whose
-  // shared-memory rows are (TX/2)*PW floats apart: with PW = 22 and TX = 16
-  // that is 176 = 16 (mod 32), so the two half-warps hit disjoint banks.
+  // Cell of this thread. For TY = 16 a warp covers two rows ROWGAP apart, so
+  // that the two half-warps of a 4-byte access to a plane (row pitch PW)
+  // hit disjoint banks: ROWGAP * PW = 16 (mod 32) words with 8 rows for
+  // PW = 22 and 4 rows for PW = 20. (8-byte accesses are served half a warp
+  // at a time.)
   int ty, tx;
-  if constexpr (TY == 16 && TX % 2 == 0) {
+  if constexpr (TY == 16 && TX % 16 == 0) {
+    constexpr int ROWGAP = PW % 8 == 4 ? 4 : 8;
     const int w = tid >> 5, lane = tid & 31;
     ty = lane & 15;
-    tx = w + (lane >> 4) * (TX / 2);
+    tx = (w / ROWGAP) * 2 * ROWGAP + w % ROWGAP + (lane >> 4) * ROWGAP;
   } else {
     ty = tid % TY;
     tx = tid / TY;
@@ -180,83 +204,98 @@ __device__ __forceinline__ void stage_body(const StageArgs& a,
   const int nxa = a.nx + 2 * h, nya = a.ny + 2 * h;
   const long long sx = a.sx, sz = a.sz;
 
-  const T* __restrict__ ukp[NCS];
-#pragma unroll
-  for (int v = 0; v < 5 + NS; ++v) ukp[v] = static_cast<const T*>(a.uk[v]);
-  if constexpr (HELP) ukp[5 + NS] = static_cast<const T*>(ext->p_ref);
   const T* __restrict__ pex = static_cast<const T*>(a.pe[0]);
   const T* __restrict__ pey = static_cast<const T*>(a.pe[1]);
   const T* __restrict__ pez = static_cast<const T*>(a.pe[2]);
   const bool has_pe = a.has_pe != 0;
 
   const T dx = T(a.dx), dy = T(a.dy), dz = T(a.dz);
-  const T nu = T(a.nu), inv_pr = T(1.0 / a.pr);
+  // Reciprocals of the launch-constant spacings.
+  const T rdx = rcp_(dx), rdy = rcp_(dy), rdz = rcp_(dz);
+  const T nu = T(a.nu);
+  const T kq = VISC ? heat_coefficient<T>(a.pr) : T(0);
 
   auto pe_at = [&](int xa, int ya, int za) -> T {
     if (!has_pe) return T(0);
-    T ax = pex ? pex[xa] : T(0);
-    T ay = pey ? pey[ya] : T(0);
-    T az = pez ? pez[za] : T(0);
-    return (-ax - ay) - az;
+    const T ax = pex ? pex[xa] : T(0);
+    const T ay = pey ? pey[ya] : T(0);
+    const T az = pez ? pez[za] : T(0);
+    return O1::sub(O1::sub(-ax, ay), az);
   };
-  auto R = [&](int slot, int v, int px, int py) -> T& {
-    return ring[((slot * NV + v) * PH + px) * PW + py];
+  // Pair j, or variable q, of plane cell `pos` in the slot at `s`.
+  auto P2 = [&](const T* s, int j, int pos) -> V2 {
+    return reinterpret_cast<const V2*>(s)[j * PS + pos];
   };
-  // Plane cells this thread stages and converts: idx = tid + k*NT.
-  auto cell_valid = [&](int idx, int& xa, int& ya) -> bool {
+  auto V1 = [&](const T* s, int q, int pos) -> T {
+    return s[L::var_off(q) + L::var_step(q) * pos];
+  };
+
+  // Plane cells this thread copies and converts: idx = tid + k*NT, at
+  // element goff[k] of a plane (negative: none).
+  long long goff[PER];
+#pragma unroll
+  for (int k = 0; k < PER; ++k) {
+    const int idx = tid + k * NT;
     const int px = idx / PW, py = idx - px * PW;
-    xa = x0 - HR + px + h;
-    ya = y0 - HR + py + h;
-    return idx < PS && xa < nxa && ya < nya;
-  };
-  auto issue_plane = [&](int z) {
+    const int xa = x0 - HR + px + h, ya = y0 - HR + py + h;
+    goff[k] = (idx < PS && xa < nxa && ya < nya) ? xa * sx + ya : -1;
+  }
+  auto issue_plane = [&](int z, int slot) {
     const long long zo = (long long)(z + h) * sz;
+    T* const s = ring + slot * SLOT;
 #pragma unroll
-    for (int k = 0; k < PER; ++k) {
-      const int idx = tid + k * NT;
-      int xa, ya;
-      if (cell_valid(idx, xa, ya)) {
-        const long long o = zo + xa * sx + ya;
+    for (int v = 0; v < 5 + NS + (HELP ? 1 : 0); ++v) {
+      // rho, rho_u, rho_v, rho_w, rho_e, scalars, p_ref.
+      constexpr int kVar[5] = {0, 2, 3, 4, 1};
+      const int q = v < 5 ? kVar[v < 5 ? v : 0] : 7 + (v - 5);
+      const T* src;
+      if (HELP && v == 5 + NS) src = static_cast<const T*>(ext->p_ref);
+      else src = static_cast<const T*>(a.uk[v]);
+      src += zo;
 #pragma unroll
-        for (int v = 0; v < NCS; ++v) cp_async(stg + v * PS + idx, ukp[v] + o);
-      }
+      for (int k = 0; k < PER; ++k)
+        if (goff[k] >= 0)
+          cp_async(s + L::var_off(q) + L::var_step(q) * (tid + k * NT),
+                   src + goff[k]);
     }
     cp_async_commit();
   };
-  // Converts this thread's staged cells into ring slot `slot` (plane z).
+  // Converts this thread's cells of plane z in place.
   auto convert_plane = [&](int z, int slot) {
+    T* const s = ring + slot * SLOT;
 #pragma unroll
     for (int k = 0; k < PER; ++k) {
       const int idx = tid + k * NT;
       if (idx >= PS) break;
-      int xa, ya;
-      T c[5] = {T(1), T(0), T(0), T(0), T(1)};
+      const bool ok = goff[k] >= 0;
+      V2 re = P2(s, 0, idx), uv = P2(s, 1, idx), wp = P2(s, 2, idx);
+      if (!ok) {
+        re = O2::splat(T(1));
+        uv = wp = O2::splat(T(0));
+      }
       T pe = T(0);
-      if (cell_valid(idx, xa, ya)) {
-#pragma unroll
-        for (int v = 0; v < 5; ++v) c[v] = stg[v * PS + idx];
-        pe = pe_at(xa, ya, z + h);
+      if (has_pe && ok) {
+        const int px = idx / PW, py = idx - px * PW;
+        pe = pe_at(x0 - HR + px + h, y0 - HR + py + h, z + h);
       }
       T u, vv, w, e, p, hh;
-      cons_to_prim(c[0], c[1], c[2], c[3], c[4], pe, u, vv, w, e, p, hh);
-      const int px = idx / PW, py = idx - px * PW;
-      R(slot, 0, px, py) = c[0];
-      R(slot, 1, px, py) = u;
-      R(slot, 2, px, py) = vv;
-      R(slot, 3, px, py) = w;
-      R(slot, 4, px, py) = e;
-      R(slot, 5, px, py) = p;
-      R(slot, 6, px, py) = hh;
+      cons_to_prim(re.x, uv.x, uv.y, wp.x, re.y, pe, u, vv, w, e, p, hh);
+      V2* const d = reinterpret_cast<V2*>(s) + idx;
+      d[0] = O2::mk(re.x, e);
+      d[PS] = O2::mk(u, vv);
+      d[2 * PS] = O2::mk(w, p);
       if constexpr (NS > 0 || HELP) {
-        const bool ok = cell_valid(idx, xa, ya);
-        const T inv = T(1) / c[0];
+        const T inv = O1::rcp(re.x);
 #pragma unroll
-        for (int k = 0; k < NS; ++k)
-          R(slot, 7 + k, px, py) = ok ? inv * stg[(5 + k) * PS + idx] : T(0);
+        for (int q = 0; q < NS; ++q) {
+          T& x = s[L::var_off(7 + q) + L::var_step(7 + q) * idx];
+          x = ok ? O1::mul(inv, x) : T(0);
+        }
         if constexpr (HELP) {
           // p_dyn = p - p_ref, zero in the halo layers beyond the grid's
           // boundary (exchange_halos with DIRICHLET 0 on all sides).
-          const int za = z + h;
+          const int px = idx / PW, py = idx - px * PW;
+          const int xa = x0 - HR + px + h, ya = y0 - HR + py + h, za = z + h;
           const bool out =
               (xa < h && ext->boundary[0][0]) ||
               (xa >= a.nx + h && ext->boundary[0][1]) ||
@@ -264,317 +303,293 @@ __device__ __forceinline__ void stage_body(const StageArgs& a,
               (ya >= a.ny + h && ext->boundary[1][1]) ||
               (za < h && ext->boundary[2][0]) ||
               (za >= a.nz + h && ext->boundary[2][1]);
-          R(slot, 7 + NS, px, py) =
-              (ok && !out) ? p - stg[(5 + NS) * PS + idx] : T(0);
+          T& x = s[L::var_off(7 + NS) + L::var_step(7 + NS) * idx];
+          x = (ok && !out) ? O1::sub(p, x) : T(0);
         }
       }
+      s[L::var_off(6) + L::var_step(6) * idx] = hh;
     }
   };
   const int zfirst = z0 - ZLO - 1;
-  auto slot_of = [&](int z) { return (z - zfirst) % RING; };
+  // Ring slot of plane zc + d (-ZLO-1 <= d <= ZHI+2) from that of plane zc.
+  auto near_slot = [&](int slot, int d) {
+    int q = slot + d;
+    if (d < 0) q = q < 0 ? q + RING : q;
+    else q = q >= RING ? q - RING : q;
+    return q;
+  };
+  static_assert(ZLO + 1 <= RING && ZHI + 2 <= RING, "near_slot range");
 
-  // ---- one face flux in the frame rotated so that the face normal is
-  // axis 0: (n, t1, t2) = x:(x,y,z), y:(y,x,z), z:(z,x,y). The same code
-  // serves all three face directions; only ring offsets differ.
-  //   off[k]   ring offset of stencil cell k (cells i-LO .. i+RI-1) of var 0
-  //   ta/tb    ring offsets of the t1-/t1+/t2-/t2+ neighbours of the cells
-  //            a = i-1 and b = i (viscous cross derivatives)
-  auto hsel = [&](int d) -> T { return d == 0 ? dx : (d == 1 ? dy : dz); };
-  // Reciprocals of the launch-constant divisors h_d and 2 h_d.
-  const T rdx = rcp_(dx), rdy = rcp_(dy), rdz = rcp_(dz);
-  const T r2dx = rcp_(T(2) * dx), r2dy = rcp_(T(2) * dy), r2dz = rcp_(T(2) * dz);
-  auto rsel = [&](int d) -> T { return d == 0 ? rdx : (d == 1 ? rdy : rdz); };
-  auto r2sel = [&](int d) -> T { return d == 0 ? r2dx : (d == 1 ? r2dy : r2dz); };
-  //   bside    EXT only: -1, or the side (0 low, 1 high) of the grid boundary
-  //            this face lies on; pidx its index in a face plane [A][B]
   constexpr int NSA = NS > 0 ? NS : 1;
-  // Every ring variable reconstructed at the ring offsets off[k]: with
-  // CELL false the face form (stencil v[i-LO..i+RI-1] of face i-1/2; lo =
-  // neg, hi = pos), with CELL true the cell form (stencil v[c-CL..c+CR]; lo
-  // = value on the cell's lower face, hi = on its upper face). vel[] maps
-  // the rotated velocity slots to ring variables. The 7 primitives run as
-  // the pairs (rho, e), (u_n, u_t1), (u_t2, p) and h alone; each pair is
-  // one two-lane instruction stream.
-  auto recon_all = [&](auto cell_tag, const int* off, const int* vel,
-                       Prim<T>& lo, Prim<T>& hi, T* phlo, T* phhi, T& pdlo,
-                       T& pdhi) {
-    constexpr bool CELL = decltype(cell_tag)::value;
-    constexpr int NK = CELL ? CW : NW;
-    using O2 = Two<T>;
-    using O1 = One<T>;
-    using V2 = typename O2::V;
-    const int va[3] = {0, vel[0], vel[2]};
-    const int vb[3] = {4, vel[1], 5};
-    V2 rl[3], rh[3];
-#pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      const T* ba = ring + va[j] * PS;
-      const T* bb = ring + vb[j] * PS;
-      V2 sv[NK];
-#pragma unroll
-      for (int k = 0; k < NK; ++k) sv[k] = O2::mk(ba[off[k]], bb[off[k]]);
-      if constexpr (CELL) recon_cell<SCHEME, O2>(sv, a.limiter, rl[j], rh[j]);
-      else recon_face<SCHEME, O2>(sv, a.limiter, rl[j], rh[j]);
-    }
-    lo.r = rl[0].x; lo.e = rl[0].y; lo.u[0] = rl[1].x;
-    lo.u[1] = rl[1].y; lo.u[2] = rl[2].x; lo.p = rl[2].y;
-    hi.r = rh[0].x; hi.e = rh[0].y; hi.u[0] = rh[1].x;
-    hi.u[1] = rh[1].y; hi.u[2] = rh[2].x; hi.p = rh[2].y;
-    auto one = [&](int var, T& l, T& r) {
-      const T* base = ring + var * PS;
-      T sv[NK];
-#pragma unroll
-      for (int k = 0; k < NK; ++k) sv[k] = base[off[k]];
-      if constexpr (CELL) recon_cell<SCHEME, O1>(sv, a.limiter, l, r);
-      else recon_face<SCHEME, O1>(sv, a.limiter, l, r);
-    };
-    one(6, lo.h, hi.h);
-#pragma unroll
-    for (int q = 0; q < NS; ++q) one(7 + q, phlo[q], phhi[q]);
-    if constexpr (HELP) {
-      one(7 + NS, pdlo, pdhi);
-    } else {
-      pdlo = lo.p;
-      pdhi = hi.p;
-    }
+  // Face values of every variable: the pairs and the last one alone.
+  struct Faces {
+    V2 q[NP];
+    T o;
   };
-  // z faces: the lower state of the face above plane zc is the upper-face
-  // value of cell zc, carried from the previous plane's reconstruction.
-  Prim<T> zq;
-  T zph[NSA], zpd;
-  auto face = [&](int dn, const int* off, int oa, int ob, const int* ta,
-                  const int* tb, T pe, int bside, long long pidx, T* f) {
-    const int t1 = dn == 0 ? 1 : 0, t2 = dn == 2 ? 1 : 2;
-    const int vel[3] = {1 + dn, 1 + t1, 1 + t2};
-    Prim<T> ql, qr;
-    T phl[NSA], phr[NSA];
-    T pdl, pdr;
-    if (dn == 2) {
-      // off[] is the cell stencil of cell zc+1: its lower-face value is the
-      // upper state of this face, its upper-face value carries on.
-      Prim<T> up;
-      T phu[NSA], pdu;
-      recon_all(std::true_type{}, off, vel, qr, up, phr, phu, pdr, pdu);
-      ql = zq;
-      zq = up;
-#pragma unroll
-      for (int q = 0; q < NS; ++q) {
-        phl[q] = zph[q];
-        zph[q] = phu[q];
-      }
-      pdl = zpd;
-      zpd = pdu;
-    } else {
-      recon_all(std::false_type{}, off, vel, ql, qr, phl, phr, pdl, pdr);
-    }
-    auto plane_val = [&](const SwcOverride& o) -> T {
-      return o.plane ? static_cast<const T*>(o.plane)[pidx] : T(o.value);
+  auto state = [&](const Faces& f, int n, Prim<T>& s, T* ph, T& pd) {
+    // Normal n, tangential t1, t2 in the rotated frame: x:(x,y,z),
+    // y:(y,x,z), z:(z,x,y).
+    const T u = f.q[1].x, v = f.q[1].y, w = f.q[2].x;
+    s.r = f.q[0].x;
+    s.e = f.q[0].y;
+    s.p = f.q[2].y;
+    s.u[0] = n == 2 ? w : (n == 0 ? u : v);
+    s.u[1] = n == 0 ? v : u;
+    s.u[2] = n == 2 ? v : w;
+    auto var = [&](int q) -> T {
+      return q / 2 < NP ? ((q & 1) ? f.q[q / 2 < NP ? q / 2 : 0].y
+                                   : f.q[q / 2 < NP ? q / 2 : 0].x)
+                        : f.o;
     };
-    if constexpr (EXT) {
-      // Face BCs on both face states (boundary.py:247-337): a primitive is
-      // set directly, a conservative one divided by the face density.
-      if (bside >= 0) {
-        const int n = ext->nface[dn][bside];
-        for (int i = 0; i < n; ++i) {
-          const SwcOverride& o = ext->face[dn][bside][i];
-          const T val = plane_val(o);
-          const bool cons = o.mode == SWC_FACE_CONSERVATIVE;
-          const T vl = cons ? dnn(val, ql.r) : val;
-          const T vr = cons ? dnn(val, qr.r) : val;
-          const int c = o.var - 1;
-          const int rr = c == dn ? 0 : (c == t1 ? 1 : 2);
+    s.h = var(6);
 #pragma unroll
-          for (int r = 0; r < 3; ++r)
-            if (o.var >= 1 && o.var <= 3 && r == rr) {
-              ql.u[r] = vl;
-              qr.u[r] = vr;
-            }
-          if (o.var == 4) {
-            ql.e = vl;
-            qr.e = vr;
-          }
-#pragma unroll
-          for (int q = 0; q < NS; ++q)
-            if (o.var == 5 + q) {
-              phl[q] = vl;
-              phr[q] = vr;
-            }
-        }
-      }
-    }
-    T g[5];
-    if constexpr (HELP) {
-      if constexpr (RIEMANN == 0) hll_flux<T, 0>(ql, qr, pdl, pdr, pe, g);
-      else hllc_flux<T, 0>(ql, qr, pdl, pdr, pe, g);
-    } else {
-      riemann<RIEMANN, T, 0>(ql, qr, pe, g);
-    }
-    T gs[NSA];
-    if constexpr (NS > 0)
-      scalar_fluxes<RIEMANN, T, 0>(ql, qr, pdl, pdr, pe, NS, phl, phr, gs);
-    // Back to (x, y, z) momentum order.
-    auto rot = [&](const T* gg, T* out) {
-      out[0] = gg[0];
-      out[1] = dn == 0 ? gg[1] : gg[2];
-      out[2] = dn == 1 ? gg[1] : (dn == 0 ? gg[2] : gg[3]);
-      out[3] = dn == 2 ? gg[1] : gg[3];
-      out[4] = gg[4];
-    };
-    // Flux BCs of one type (boundary.py:89-183) on fb (x, y, z order) and
-    // the scalar fluxes fbs.
-    auto flux_bc = [&](int type, T* fb, T* fbs) {
-      if (bside < 0) return;
-      const int n = ext->nflux[dn][bside];
-      for (int i = 0; i < n; ++i) {
-        const SwcOverride& o = ext->flux[dn][bside][i];
-        if (o.mode != type) continue;
-        const T val = plane_val(o);
-#pragma unroll
-        for (int v = 0; v < 5; ++v)
-          if (o.var == v) fb[v] = val;
-#pragma unroll
-        for (int q = 0; q < NS; ++q)
-          if (o.var == 5 + q) fbs[q] = val;
-      }
-    };
-    if constexpr (EXT) {
-      T fc[5];
-      rot(g, fc);
-      flux_bc(SWC_FLUX_CONVECTIVE, fc, gs);
-      T fv[5] = {T(0), T(0), T(0), T(0), T(0)};
-      T fvs[NSA];
-#pragma unroll
-      for (int q = 0; q < NSA; ++q) fvs[q] = T(0);
-      if constexpr (VISC) {
-        T gv[5] = {T(0), T(0), T(0), T(0), T(0)};
-        T ua[3], ub[3], ga[3][3], gb[3][3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          ua[c] = ring[vel[c] * PS + oa];
-          ub[c] = ring[vel[c] * PS + ob];
-        }
-        const T i2t1 = T(2) * hsel(t1), i2t2 = T(2) * hsel(t2);
-        const T ri2t1 = r2sel(t1), ri2t2 = r2sel(t2);
-        ga[1][1] = divk(ring[vel[1] * PS + ta[1]] - ring[vel[1] * PS + ta[0]], i2t1, ri2t1);
-        gb[1][1] = divk(ring[vel[1] * PS + tb[1]] - ring[vel[1] * PS + tb[0]], i2t1, ri2t1);
-        ga[1][0] = divk(ring[vel[0] * PS + ta[1]] - ring[vel[0] * PS + ta[0]], i2t1, ri2t1);
-        gb[1][0] = divk(ring[vel[0] * PS + tb[1]] - ring[vel[0] * PS + tb[0]], i2t1, ri2t1);
-        ga[2][2] = divk(ring[vel[2] * PS + ta[3]] - ring[vel[2] * PS + ta[2]], i2t2, ri2t2);
-        gb[2][2] = divk(ring[vel[2] * PS + tb[3]] - ring[vel[2] * PS + tb[2]], i2t2, ri2t2);
-        ga[2][0] = divk(ring[vel[0] * PS + ta[3]] - ring[vel[0] * PS + ta[2]], i2t2, ri2t2);
-        gb[2][0] = divk(ring[vel[0] * PS + tb[3]] - ring[vel[0] * PS + tb[2]], i2t2, ri2t2);
-        viscous_flux<T, 0>(ring[oa], ring[ob], ua, ub, ring[5 * PS + oa],
-                           ring[5 * PS + ob], ga, gb, hsel(dn), rsel(dn), nu,
-                           inv_pr, gv);
-        rot(gv, fv);
-        flux_bc(SWC_FLUX_DIFFUSIVE, fv, fvs);
-      }
-#pragma unroll
-      for (int v = 0; v < 5; ++v) f[v] = fc[v] + fv[v];
-#pragma unroll
-      for (int q = 0; q < NS; ++q) f[5 + q] = gs[q] + fvs[q];
-      flux_bc(SWC_FLUX_TOTAL, f, f + 5);
-      return;
-    }
-    if constexpr (VISC) {
-      T ua[3], ub[3], ga[3][3], gb[3][3];
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        ua[c] = ring[vel[c] * PS + oa];
-        ub[c] = ring[vel[c] * PS + ob];
-      }
-      const T i2t1 = T(2) * hsel(t1), i2t2 = T(2) * hsel(t2);
-      const T ri2t1 = r2sel(t1), ri2t2 = r2sel(t2);
-      // Along t1: components t1 (rotated 1) and n (rotated 0).
-      ga[1][1] = divk(ring[vel[1] * PS + ta[1]] - ring[vel[1] * PS + ta[0]], i2t1, ri2t1);
-      gb[1][1] = divk(ring[vel[1] * PS + tb[1]] - ring[vel[1] * PS + tb[0]], i2t1, ri2t1);
-      ga[1][0] = divk(ring[vel[0] * PS + ta[1]] - ring[vel[0] * PS + ta[0]], i2t1, ri2t1);
-      gb[1][0] = divk(ring[vel[0] * PS + tb[1]] - ring[vel[0] * PS + tb[0]], i2t1, ri2t1);
-      // Along t2: components t2 (rotated 2) and n.
-      ga[2][2] = divk(ring[vel[2] * PS + ta[3]] - ring[vel[2] * PS + ta[2]], i2t2, ri2t2);
-      gb[2][2] = divk(ring[vel[2] * PS + tb[3]] - ring[vel[2] * PS + tb[2]], i2t2, ri2t2);
-      ga[2][0] = divk(ring[vel[0] * PS + ta[3]] - ring[vel[0] * PS + ta[2]], i2t2, ri2t2);
-      gb[2][0] = divk(ring[vel[0] * PS + tb[3]] - ring[vel[0] * PS + tb[2]], i2t2, ri2t2);
-      viscous_flux<T, 0>(ring[oa], ring[ob], ua, ub, ring[5 * PS + oa],
-                         ring[5 * PS + ob], ga, gb, hsel(dn), rsel(dn), nu,
-                         inv_pr, g);
-    }
-    rot(g, f);
-#pragma unroll
-    for (int q = 0; q < NS; ++q) f[5 + q] = gs[q];
+    for (int k = 0; k < NS; ++k) ph[k] = var(7 + k);
+    pd = HELP ? var(7 + NS) : s.p;
   };
 
-  const int SL = NV * PS;  // ring slot stride
+  // Face BCs on both face states (boundary.py:247-337): a primitive is set
+  // directly, a conservative one divided by the face density. Flux BCs of
+  // one type (boundary.py:89-183). dn: face normal; bside: -1, or the side
+  // (0 low, 1 high) of the grid boundary the face lies on; pidx: its index
+  // in a face plane [A][B].
+  auto plane_val = [&](const SwcOverride& o, long long pidx) -> T {
+    return o.plane ? static_cast<const T*>(o.plane)[pidx] : T(o.value);
+  };
+  auto face_bc = [&](int dn, int bside, long long pidx, Prim<T>& l,
+                     Prim<T>& r, T* phl, T* phr) {
+    const int t1 = dn == 0 ? 1 : 0;
+    const int n = ext->nface[dn][bside];
+    for (int i = 0; i < n; ++i) {
+      const SwcOverride& o = ext->face[dn][bside][i];
+      const T val = plane_val(o, pidx);
+      const bool cons = o.mode == SWC_FACE_CONSERVATIVE;
+      const T vl = cons ? dnn(val, l.r) : val;
+      const T vr = cons ? dnn(val, r.r) : val;
+      const int c = o.var - 1;
+      const int rr = c == dn ? 0 : (c == t1 ? 1 : 2);
+#pragma unroll
+      for (int q = 0; q < 3; ++q)
+        if (o.var >= 1 && o.var <= 3 && q == rr) {
+          l.u[q] = vl;
+          r.u[q] = vr;
+        }
+      if (o.var == 4) {
+        l.e = vl;
+        r.e = vr;
+      }
+#pragma unroll
+      for (int q = 0; q < NS; ++q)
+        if (o.var == 5 + q) {
+          phl[q] = vl;
+          phr[q] = vr;
+        }
+    }
+  };
+  auto flux_bc = [&](int dn, int bside, long long pidx, int type, T* fb) {
+    const int n = ext->nflux[dn][bside];
+    for (int i = 0; i < n; ++i) {
+      const SwcOverride& o = ext->flux[dn][bside][i];
+      if (o.mode != type) continue;
+      const T val = plane_val(o, pidx);
+#pragma unroll
+      for (int v = 0; v < NF; ++v)
+        if (o.var == v) fb[v] = val;
+    }
+  };
+  // Total flux (x, y, z momentum order, then scalars) from the face states
+  // and the viscous flux v (rotated, VISC only).
+  auto flux = [&](int dn, const Faces& lo, const Faces& hi, T pe, const T* v,
+                  int bside, long long pidx, T* f) {
+    Prim<T> l, r;
+    T phl[NSA], phr[NSA], pdl, pdr, g[5], gs[NSA];
+    state(lo, dn, l, phl, pdl);
+    state(hi, dn, r, phr, pdr);
+    if constexpr (EXT)
+      if (bside >= 0) face_bc(dn, bside, pidx, l, r, phl, phr);
+    if constexpr (!HELP) {
+      pdl = l.p;
+      pdr = r.p;
+    }
+    face_flux<RIEMANN, T, 0, NS>(l, r, pdl, pdr, pe, phl, phr, g, gs);
+    auto rot = [&](T n, T a1, T a2, T* out) {
+      out[1] = dn == 0 ? n : a1;
+      out[2] = dn == 1 ? n : (dn == 0 ? a1 : a2);
+      out[3] = dn == 2 ? n : a2;
+    };
+    if constexpr (EXT) {
+      f[0] = g[0];
+      rot(g[1], g[2], g[3], f);
+      f[4] = g[4];
+#pragma unroll
+      for (int k = 0; k < NS; ++k) f[5 + k] = gs[k];
+      if (bside >= 0) flux_bc(dn, bside, pidx, SWC_FLUX_CONVECTIVE, f);
+      T fv[NF];
+#pragma unroll
+      for (int k = 0; k < NF; ++k) fv[k] = T(0);
+      if constexpr (VISC) {
+        rot(v[0], v[1], v[2], fv);
+        fv[4] = v[3];
+        if (bside >= 0) flux_bc(dn, bside, pidx, SWC_FLUX_DIFFUSIVE, fv);
+      }
+#pragma unroll
+      for (int k = 0; k < NF; ++k) f[k] = O1::add(f[k], fv[k]);
+      if (bside >= 0) flux_bc(dn, bside, pidx, SWC_FLUX_TOTAL, f);
+    } else {
+      if constexpr (VISC) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) g[1 + k] = O1::add(g[1 + k], v[k]);
+      }
+      f[0] = g[0];
+      rot(g[1], g[2], g[3], f);
+      f[4] = g[4];
+#pragma unroll
+      for (int k = 0; k < NS; ++k) f[5 + k] = gs[k];
+    }
+  };
+  // Grid-boundary side of the face normal to `dn` stored at index i of n
+  // (face i-1/2: i = 0 is the low boundary, i = n the high one,
+  // boundary.py:140-183).
+  auto side_of = [&](int dn, int i, int n) -> int {
+    int b = -1;
+    if constexpr (EXT) {
+      if (i == 0 && ext->boundary[dn][0]) b = 0;
+      if (i == n && ext->boundary[dn][1]) b = 1;
+    }
+    return b;
+  };
+
   // Flux buffers of the plane in progress, and this thread's z-face flux.
   T* fx = fx0;
   T* fy = fy0;
   T fzr[NF];
-  // Face of kind `kind` (0 = x-face at row fxx, 1 = y-face at column fyy,
-  // 2 = z-face above plane zc) into the flux buffers (z: into fzr).
-  auto do_face = [&](int kind, int zc, int fxx, int fyy) {
-    int off[NOFF], ta[4], tb[4];
-    T pe;
-    T f[NF];
-    // Grid-boundary side and face-plane index of this face (EXT only). The
-    // face stored at i (interior numbering) is face i-1/2: i = 0 is the low
-    // boundary, i = n the high one (boundary.py:140-183).
+  // x (isx) or y face at row fxx, column fyy of plane zc, in slot sc, into
+  // the flux buffers. One copy of the code serves both axes: only the
+  // stencil's stride and the order of u and v differ.
+  auto face_xy = [&](bool isx, int zc, int sc, int fxx, int fyy) {
+    const int dn = isx ? 0 : 1;
+    const int pos = (HR + fxx) * PW + HR + fyy;
+    const int st = isx ? PW : 1;
+    const T* const s = ring + sc * SLOT;
+    T fv[4];
+    if constexpr (VISC) {
+      // Cells a = i-1, b = i; t1 is the other in-plane axis, t2 is z.
+      const int s1 = isx ? 1 : PW;
+      const int pa = pos - st, pb = pos;
+      const T r1 = O1::mul(T(0.25), isx ? rdy : rdx);
+      const T r2 = O1::mul(T(0.25), rdz);
+      const V2 d1 = O2::add(O2::sub(P2(s, 1, pa + s1), P2(s, 1, pa - s1)),
+                            O2::sub(P2(s, 1, pb + s1), P2(s, 1, pb - s1)));
+      const T* const su = ring + near_slot(sc, 1) * SLOT;
+      const T* const sd = ring + near_slot(sc, -1) * SLOT;
+      const int vn = (isx ? L::var_off(2) : L::var_off(3));
+      auto dz4 = [&](int off) -> T {
+        return O1::add(O1::sub(su[off + 2 * pa], sd[off + 2 * pa]),
+                       O1::sub(su[off + 2 * pb], sd[off + 2 * pb]));
+      };
+      const T g11 = O1::mul(isx ? d1.y : d1.x, r1);
+      const T g10 = O1::mul(isx ? d1.x : d1.y, r1);
+      const T g22 = O1::mul(dz4(L::var_off(4)), r2);
+      const T g20 = O1::mul(dz4(vn), r2);
+      const V2 ua2 = P2(s, 1, pa), ub2 = P2(s, 1, pb);
+      const V2 wa = P2(s, 2, pa), wb = P2(s, 2, pb);
+      const T ua[3] = {isx ? ua2.x : ua2.y, isx ? ua2.y : ua2.x, wa.x};
+      const T ub[3] = {isx ? ub2.x : ub2.y, isx ? ub2.y : ub2.x, wb.x};
+      viscous_flux<T>(V1(s, 0, pa), V1(s, 0, pb), ua, ub, wa.y, wb.y, g11, g10,
+                      g22, g20, isx ? rdx : rdy, nu, kq, fv);
+    }
+    Faces lo, hi;
+#pragma unroll
+    for (int j = 0; j < NP; ++j) {
+      V2 sv[NW];
+#pragma unroll
+      for (int k = 0; k < NW; ++k) sv[k] = P2(s, j, pos + (k - LO) * st);
+      recon_face<SCHEME, O2>(sv, a.limiter, lo.q[j], hi.q[j]);
+    }
+    if constexpr (NV & 1) {
+      T sv[NW];
+#pragma unroll
+      for (int k = 0; k < NW; ++k) sv[k] = V1(s, NV - 1, pos + (k - LO) * st);
+      recon_face<SCHEME, O1>(sv, a.limiter, lo.o, hi.o);
+    }
+    const T pe = pe_at(x0 + fxx + h, y0 + fyy + h, zc + h);
     int bside = -1;
     long long pidx = 0;
     if constexpr (EXT) {
-      const int i = kind == 0 ? x0 + fxx : (kind == 1 ? y0 + fyy : zc + 1);
-      const int n = kind == 0 ? a.nx : (kind == 1 ? a.ny : a.nz);
-      if (i == 0 && ext->boundary[kind][0]) bside = 0;
-      if (i == n && ext->boundary[kind][1]) bside = 1;
-      if (kind == 0) pidx = (long long)(zc + h) * nya + (y0 + fyy + h);
-      else if (kind == 1) pidx = (long long)(zc + h) * nxa + (x0 + fxx + h);
-      else pidx = (long long)(x0 + fxx + h) * nya + (y0 + fyy + h);
+      bside = isx ? side_of(0, x0 + fxx, a.nx) : side_of(1, y0 + fyy, a.ny);
+      pidx = isx ? (long long)(zc + h) * nya + (y0 + fyy + h)
+                 : (long long)(zc + h) * nxa + (x0 + fxx + h);
     }
-    if (kind == 2) {
-      const int pos = (HR + fxx) * PW + HR + fyy;
+    T f[NF];
+    flux(dn, lo, hi, pe, fv, bside, pidx, f);
+    T* const buf = isx ? fx : fy;
+    const int n = isx ? L::NX : L::NY;
+    const int p = isx ? fxx * TY + fyy : fxx * (TY + 1) + fyy;
+    V2* const b2 = reinterpret_cast<V2*>(buf) + p;
+    b2[0] = O2::mk(f[0], f[4]);
+    b2[n] = O2::mk(f[1], f[2]);
 #pragma unroll
-      for (int k = 0; k < CW; ++k) off[k] = slot_of(zc + 1 - CL + k) * SL + pos;
-      const int oa = slot_of(zc) * SL + pos, ob = slot_of(zc + 1) * SL + pos;
-      ta[0] = oa - PW; ta[1] = oa + PW; ta[2] = oa - 1; ta[3] = oa + 1;
-      tb[0] = ob - PW; tb[1] = ob + PW; tb[2] = ob - 1; tb[3] = ob + 1;
-      pe = pe_at(x0 + fxx + h, y0 + fyy + h, zc + 1 + h);
-      face(2, off, oa, ob, ta, tb, pe, bside, pidx, f);
+    for (int j = 2; j < NFP; ++j) {
+      const int c = 2 * j;  // components (3, 5), (6, 7)
+      b2[j * n] = O2::mk(c == 4 ? f[3] : f[c], f[c + 1 < NF ? c + 1 : 0]);
+    }
+    if constexpr (NF & 1) buf[2 * NFP * n + p] = f[NF == 5 ? 3 : NF - 1];
+  };
+  // z-face above plane zc (slot sc), into fzr. The cell above it (zc+1) is
+  // reconstructed along z: its lower-face value is this face's upper state,
+  // its upper-face value the next face's lower state, carried in zq.
+  Faces zq;
+  auto recon_z = [&](const int* sl, int pos, Faces& lo, Faces& hi) {
 #pragma unroll
-      for (int v = 0; v < NF; ++v) fzr[v] = f[v];
-    } else {
-      const int cs = slot_of(zc) * SL;
-      const int dm = (slot_of(zc - 1) - slot_of(zc)) * SL;
-      const int dp = (slot_of(zc + 1) - slot_of(zc)) * SL;
-      const int pos = cs + (HR + fxx) * PW + HR + fyy;
-      const int st = kind == 0 ? PW : 1;     // normal stride
-      const int s1 = kind == 0 ? 1 : PW;     // t1 stride (y for x-faces, x for y-faces)
+    for (int j = 0; j < NP; ++j) {
+      V2 sv[CW];
 #pragma unroll
-      for (int k = 0; k < NW; ++k) off[k] = pos + (k - LO) * st;
-      const int oa = pos - st, ob = pos;
-      ta[0] = oa - s1; ta[1] = oa + s1; ta[2] = oa + dm; ta[3] = oa + dp;
-      tb[0] = ob - s1; tb[1] = ob + s1; tb[2] = ob + dm; tb[3] = ob + dp;
-      pe = pe_at(x0 + fxx + h, y0 + fyy + h, zc + h);
-      face(kind, off, oa, ob, ta, tb, pe, bside, pidx, f);
-      if (kind == 0) {
+      for (int k = 0; k < CW; ++k) sv[k] = P2(ring + sl[k], j, pos);
+      recon_cell<SCHEME, O2>(sv, a.limiter, lo.q[j], hi.q[j]);
+    }
+    if constexpr (NV & 1) {
+      T sv[CW];
 #pragma unroll
-        for (int v = 0; v < NF; ++v) fx[(v * (TX + 1) + fxx) * TY + fyy] = f[v];
-      } else {
-#pragma unroll
-        for (int v = 0; v < NF; ++v) fy[(v * TX + fxx) * (TY + 1) + fyy] = f[v];
-      }
+      for (int k = 0; k < CW; ++k) sv[k] = V1(ring + sl[k], NV - 1, pos);
+      recon_cell<SCHEME, O1>(sv, a.limiter, lo.o, hi.o);
     }
   };
+  auto face_z = [&](int zc, int sc) {
+    const int pos = (HR + tx) * PW + HR + ty;
+    T fv[4];
+    if constexpr (VISC) {
+      const T* const sa = ring + sc * SLOT;
+      const T* const sb = ring + near_slot(sc, 1) * SLOT;
+      const T r1 = O1::mul(T(0.25), rdx), r2 = O1::mul(T(0.25), rdy);
+      auto diff = [&](int q, int st) -> T {
+        return O1::add(O1::sub(V1(sa, q, pos + st), V1(sa, q, pos - st)),
+                       O1::sub(V1(sb, q, pos + st), V1(sb, q, pos - st)));
+      };
+      const T g11 = O1::mul(diff(2, PW), r1), g10 = O1::mul(diff(4, PW), r1);
+      const T g22 = O1::mul(diff(3, 1), r2), g20 = O1::mul(diff(4, 1), r2);
+      const V2 ua2 = P2(sa, 1, pos), ub2 = P2(sb, 1, pos);
+      const V2 wa = P2(sa, 2, pos), wb = P2(sb, 2, pos);
+      const T ua[3] = {wa.x, ua2.x, ua2.y}, ub[3] = {wb.x, ub2.x, ub2.y};
+      viscous_flux<T>(V1(sa, 0, pos), V1(sb, 0, pos), ua, ub, wa.y, wb.y, g11,
+                      g10, g22, g20, rdz, nu, kq, fv);
+    }
+    int sl[CW];
+#pragma unroll
+    for (int k = 0; k < CW; ++k) sl[k] = near_slot(sc, 1 - CL + k) * SLOT;
+    Faces lo, up;
+    recon_z(sl, pos, lo, up);
+    const T pe = pe_at(x0 + tx + h, y0 + ty + h, zc + 1 + h);
+    flux(2, zq, lo, pe, fv, side_of(2, zc + 1, a.nz),
+         (long long)(x0 + tx + h) * nya + (y0 + ty + h), fzr);
+    zq = up;
+  };
 
-  // ---- warm-up: planes zfirst .. z0+ZHI-1 through the staging buffer (the
-  // ring of the loop's first pass, zc = z0-1, which only computes the z-face
-  // below the segment, so that every face of every segment comes from the
-  // same code: results do not depend on where segments start); plane
-  // z0+ZHI, converted during that pass, in flight.
-  for (int i = 0; i < RING - SPARE; ++i) {
-    issue_plane(zfirst + i);
-    cp_async_wait_all();
-    convert_plane(zfirst + i, i);
-  }
-  if (z0 < z1) issue_plane(z0 + ZHI);
+  // ---- warm-up: planes zfirst .. z0+ZHI-1, all copies in flight at once
+  // (the ring of the loop's first pass, zc = z0-1, which only computes the
+  // z-face below the segment, so that every face of every segment comes from
+  // the same code: results do not depend on where segments start).
+  for (int i = 0; i < RING - SPARE; ++i) issue_plane(zfirst + i, i);
+  cp_async_wait_all();
+  for (int i = 0; i < RING - SPARE; ++i) convert_plane(zfirst + i, i);
   __syncthreads();
   const bool own = (x0 + tx < a.nx) && (y0 + ty < a.ny);
   T flo[NF];
@@ -595,7 +610,6 @@ __device__ __forceinline__ void stage_body(const StageArgs& a,
   static_assert(NT % 32 == 0, "whole warps");
   constexpr int NWARP = NT / 32;
   const int tile_rot = x0 / TX + y0 / TY;
-  const int nj = own ? 3 : 0;
   int bkind = -1, bx = 0, by = 0;
   auto boundary_faces = [&](int zc) {
     int wb = tid - ((zc - z0 + tile_rot) % NWARP) * 32;
@@ -612,63 +626,67 @@ __device__ __forceinline__ void stage_body(const StageArgs& a,
   const bool ex_y = own && (y0 + ty + 1 == a.ny) && (ty + 1 < TY);
 
   // One barrier per plane: faces of plane zc (x and y into flux buffer
-  // zc & 1, z into registers), then the conversion of plane zc+ZHI+1 into
-  // a slot no face of plane zc reads, the barrier, and the update of plane
-  // zc, which reads no ring slot. A thread may start the faces of plane
-  // zc+1 while others still update plane zc: they write the other flux
+  // zc & 1, z into registers), then the in-place conversion of plane
+  // zc+ZHI+1 in a slot no face of plane zc reads, the barrier, and the update
+  // of plane zc, which reads no ring slot. A thread may start the faces of
+  // plane zc+1 while others still update plane zc: they write the other flux
   // buffer, and buffer zc & 1 is next written after the following barrier.
-  for (int zc = z0 - 1; zc < z1; ++zc) {
+  // The copy of plane zc+ZHI+2 starts after that barrier, into the slot of
+  // plane zc+1-ZLO-SPARE: the faces of plane zc were its last readers.
+  int sc = ZLO;  // slot of plane zc
+  for (int zc = z0 - 1; zc < z1; ++zc, sc = near_slot(sc, 1)) {
     const bool pre = zc < z0;  // only the z-face below the segment
     fx = fx0 + ((zc - z0 + 1) & 1) * L::FX_ELEMS;
     fy = fy0 + ((zc - z0 + 1) & 1) * L::FY_ELEMS;
-    if (pre && own) {
-      // Upper-face value of cell z0-1: the lower state of the segment's
-      // first z face.
-      const int pos = (HR + tx) * PW + HR + ty;
-      int off[CW];
+    if (pre) {
+      if (own) {
+        // Upper-face value of cell z0-1: the lower state of the segment's
+        // first z face.
+        int sl[CW];
 #pragma unroll
-      for (int k = 0; k < CW; ++k) off[k] = slot_of(zc - CL + k) * SL + pos;
-      const int vel[3] = {3, 1, 2};
-      Prim<T> lf;
-      T phlf[NSA], pdlf;
-      recon_all(std::true_type{}, off, vel, lf, zq, phlf, zph, pdlf, zpd);
+        for (int k = 0; k < CW; ++k) sl[k] = near_slot(sc, -CL + k) * SLOT;
+        Faces lf;
+        recon_z(sl, (HR + tx) * PW + HR + ty, lf, zq);
+      }
+      // The first pass reads plane zc-CL, whose slot the next plane may
+      // take: every thread has read it before the copy starts.
+      __syncthreads();
+      if (zc + 1 < z1) issue_plane(zc + ZHI + 1, near_slot(sc, ZHI + 1));
+    } else {
+      boundary_faces(zc);
     }
-    if (!pre) boundary_faces(zc);
-    const int ntot = pre ? (own ? 1 : 0) : nj + (bkind >= 0) + ex_x + ex_y;
-    for (int j = 0; j < ntot; ++j) {
-      int kind, fxx, fyy;
-      if (j < nj) {
-        kind = 2 - j;  // z, y, x
-        fxx = tx;
-        fyy = ty;
+    if (own) face_z(zc, sc);
+    const int nxy = pre ? 0 : (own ? 2 : 0) + (bkind >= 0) + ex_x + ex_y;
+#pragma unroll 1
+    for (int j = 0; j < nxy; ++j) {
+      bool isx;
+      int fxx = tx, fyy = ty;
+      int e = j - (own ? 2 : 0);
+      if (e < 0) {
+        isx = j == 1;  // y, x
       } else {
-        int e = j - nj;
         if (bkind >= 0 && e == 0) {
-          kind = bkind; fxx = bx; fyy = by;
+          isx = bkind == 0; fxx = bx; fyy = by;
         } else {
           if (bkind >= 0) --e;
-          if (e == 0 && ex_x) { kind = 0; fxx = tx + 1; fyy = ty; }
-          else { kind = 1; fxx = tx; fyy = ty + 1; }
+          isx = e == 0 && ex_x;
+          if (isx) fxx = tx + 1;
+          else fyy = ty + 1;
         }
       }
-      do_face(kind, zc, fxx, fyy);
+      face_xy(isx, zc, sc, fxx, fyy);
     }
     // The cell's density for the gravity source, read while plane zc's
     // slot is certain to hold it (before the barrier).
-    const T rho_cell =
-        (a.gravity_mask && own && !pre) ? R(slot_of(zc), 0, HR + tx, HR + ty)
-                                        : T(0);
-    // Plane zc+ZHI+1 (staged during the previous plane) replaces the slot
-    // of plane zc-ZLO-SPARE, which no face of plane zc reads. The first
-    // pass also read plane zc-CL (its own cell's reconstruction), which can
-    // be that plane: there the other threads' reads are waited for first.
+    const T rho_cell = (a.gravity_mask && own && !pre)
+                           ? V1(ring + sc * SLOT, 0, (HR + tx) * PW + HR + ty)
+                           : T(0);
     if (zc + 1 < z1) {
-      if (pre) __syncthreads();
       cp_async_wait_all();
-      convert_plane(zc + ZHI + 1, slot_of(zc + ZHI + 1));
-      if (zc + 2 < z1) issue_plane(zc + ZHI + 2);
+      convert_plane(zc + ZHI + 1, near_slot(sc, ZHI + 1));
     }
     __syncthreads();
+    if (zc + 2 < z1) issue_plane(zc + ZHI + 2, near_slot(sc, ZHI + 2));
     if (pre) {
       if (own) {
 #pragma unroll
@@ -684,7 +702,7 @@ __device__ __forceinline__ void stage_body(const StageArgs& a,
       T ukc[NF], u0c[NF];
 #pragma unroll
       for (int v = 0; v < NF; ++v) {
-        ukc[v] = __ldg(ukp[v] + o);
+        ukc[v] = __ldg(static_cast<const T*>(a.uk[v]) + o);
         u0c[v] = (a.mode >= SWC_OUT_CONVEX)
                      ? __ldg(static_cast<const T*>(a.u0[v]) + o)
                      : T(0);
@@ -700,26 +718,43 @@ __device__ __forceinline__ void stage_body(const StageArgs& a,
           if (a.gravity_mask & (1 << d))
             src[1 + d] = rho_c * K<T>::grav() * T(a.g[d]);
       }
+      // Flux differences over the cell, component order (0, 4), (1, 2),
+      // (3, 5), (6, 7).
+      T ddx[NF], ddy[NF];
+      const int px = tx * TY + ty, py = tx * (TY + 1) + ty;
+      auto diffs = [&](const T* buf, int n, int p, int step, T* d) {
+        const V2* const b2 = reinterpret_cast<const V2*>(buf) + p;
+#pragma unroll
+        for (int j = 0; j < NFP; ++j) {
+          const V2 t = O2::sub(b2[j * n + step], b2[j * n]);
+          const int c = 2 * j;
+          d[c == 0 ? 0 : (c == 2 ? 1 : (c == 4 ? 3 : c))] = t.x;
+          d[c == 0 ? 4 : (c == 2 ? 2 : (c + 1 < NF ? c + 1 : 0))] = t.y;
+        }
+        if constexpr (NF & 1)
+          d[NF == 5 ? 3 : NF - 1] = O1::sub(buf[2 * NFP * n + p + step],
+                                            buf[2 * NFP * n + p]);
+      };
+      diffs(fx, L::NX, px, TY, ddx);
+      diffs(fy, L::NY, py, 1, ddy);
       T out[NF];
 #pragma unroll
       for (int v = 0; v < NF; ++v) {
         const T fhi = fzr[v];
         T rhs = v < 5 ? src[v] : T(0);
-        rhs = rhs - divk((fx[(v * (TX + 1) + tx + 1) * TY + ty] -
-                     fx[(v * (TX + 1) + tx) * TY + ty]), dx, rdx);
-        rhs = rhs - divk((fy[(v * TX + tx) * (TY + 1) + ty + 1] -
-                     fy[(v * TX + tx) * (TY + 1) + ty]), dy, rdy);
-        rhs = rhs - divk(fhi - flo[v], dz, rdz);
+        rhs = O1::fma(-ddx[v], rdx, rhs);
+        rhs = O1::fma(-ddy[v], rdy, rhs);
+        rhs = O1::fma(-O1::sub(fhi, flo[v]), rdz, rhs);
         flo[v] = fhi;
         T r;
         if (a.mode == SWC_OUT_RHS) {
           r = rhs;
         } else if (a.mode == SWC_OUT_EULER) {
-          r = ukc[v] + rhs * dt;
+          r = O1::fma(rhs, dt, ukc[v]);
         } else if (a.mode == SWC_OUT_CONVEX) {
-          r = u0c[v] * c0 + (ukc[v] + rhs * dt) * c1;
+          r = O1::fma(O1::fma(rhs, dt, ukc[v]), c1, O1::mul(u0c[v], c0));
         } else {
-          r = c0 * (u0c[v] + (ukc[v] + dt * rhs));
+          r = O1::mul(c0, O1::add(u0c[v], O1::fma(dt, rhs, ukc[v])));
         }
         out[v] = r;
       }
@@ -736,7 +771,6 @@ __device__ __forceinline__ void stage_body(const StageArgs& a,
       }
     }
   }
-  cp_async_wait_all();
 
   if (a.dtmin_out) {
     // Block min of the CFL limits, then one atomic per CTA.
