@@ -418,6 +418,46 @@ __global__ void viscous_terms_kernel(const ViscArgs a) {
   }
 }
 
+// SMs of the current device (queried once per device).
+static int sm_count() {
+  static int cached[64] = {0};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+  if (!cached[dev]) {
+    int n = 0;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)
+      n = 148;
+    cached[dev] = n;
+  }
+  return cached[dev];
+}
+
+// Automatic z segment of the stage kernel for `tiles2d` (y, x) tiles and
+// `per_sm` resident CTAs per SM. A CTA's time is about (zseg + 1) planes
+// (the extra plane: warm-up and the z face below the segment), and the
+// launch takes ceil(CTAs / slots) rounds of them, so the segment count that
+// minimises rounds x (zseg + 1) is taken: at 256^3 that is 8 segments of 32
+// planes (7 rounds of 2048 CTAs on 296 slots) rather than a last round that
+// leaves most SMs idle.
+int auto_zseg(long long tiles2d, int nz, int per_sm) {
+  const long long slots = (long long)sm_count() * per_sm;
+  long long best_cost = -1;
+  int best = nz;
+  for (int nseg = 1; nseg <= nz; ++nseg) {
+    const int zs = (nz + nseg - 1) / nseg;
+    if (nseg > 1 && zs == (nz + nseg - 2) / (nseg - 1)) continue;  // same zseg
+    if (zs < 4 && nseg > 1) break;
+    const long long segs = (nz + zs - 1) / zs;
+    const long long rounds = (tiles2d * segs + slots - 1) / slots;
+    const long long cost = rounds * (zs + 1);
+    if (best_cost < 0 || cost < best_cost) {
+      best_cost = cost;
+      best = zs;
+    }
+  }
+  return best;
+}
+
 }  // namespace swc
 
 using namespace swc;
@@ -585,51 +625,10 @@ int swc_halo_fill(const SwcGrid* grid, int32_t dtype, int32_t nfields,
   return SWC_OK;
 }
 
-// SMs of the current device (queried once per device).
-static int sm_count() {
-  static int cached[64] = {0};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
-  if (!cached[dev]) {
-    int n = 0;
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)
-      n = 148;
-    cached[dev] = n;
-  }
-  return cached[dev];
-}
-
-// Automatic z segment of the stage kernel for `tiles2d` (y, x) tiles and
-// `per_sm` resident CTAs per SM. A CTA's time is about (zseg + 1) planes
-// (the extra plane: warm-up and the z face below the segment), and the
-// launch takes ceil(CTAs / slots) rounds of them, so the segment count that
-// minimises rounds x (zseg + 1) is taken: at 256^3 that is 8 segments of 32
-// planes (7 rounds of 2048 CTAs on 296 slots) rather than a last round that
-// leaves most SMs idle.
-static int auto_zseg(long long tiles2d, int nz, int per_sm) {
-  const long long slots = (long long)sm_count() * per_sm;
-  long long best_cost = -1;
-  int best = nz;
-  for (int nseg = 1; nseg <= nz; ++nseg) {
-    const int zs = (nz + nseg - 1) / nseg;
-    if (nseg > 1 && zs == (nz + nseg - 2) / (nseg - 1)) continue;  // same zseg
-    if (zs < 4 && nseg > 1) break;
-    const long long segs = (nz + zs - 1) / zs;
-    const long long rounds = (tiles2d * segs + slots - 1) / slots;
-    const long long cost = rounds * (zs + 1);
-    if (best_cost < 0 || cost < best_cost) {
-      best_cost = cost;
-      best = zs;
-    }
-  }
-  return best;
-}
-
 // Checks and the kernel arguments shared by swc_rk_stage and
-// swc_rk_stage_ext; `nf` conserved fields (5 + scalars); `per_sm` resident
-// CTAs per SM and the tile's ty extent (x extent 16) size the z segments.
+// swc_rk_stage_ext; `nf` conserved fields (5 + scalars). a.zseg stays 0 where
+// the launch chooses it.
 static int stage_args(const SwcGrid* grid, const SwcScheme* sc, int nf,
-                      int per_sm, int ty,
                       const void* const* uk, const void* const* u0,
                       void* const* uout, int32_t mode, double c0, double c1,
                       const double* dt, double* dtmin_out, StageArgs& a) {
@@ -674,13 +673,7 @@ static int stage_args(const SwcGrid* grid, const SwcScheme* sc, int nf,
   a.limiter = sc->limiter;
   a.nu = sc->nu; a.pr = sc->pr > 0 ? sc->pr : 1.0;
   a.gravity_mask = sc->gravity_mask;
-  int zseg = sc->zseg;
-  if (zseg <= 0) {
-    const long long tiles2d =
-        (long long)((grid->ny + ty - 1) / ty) * ((grid->nx + 15) / 16);
-    zseg = auto_zseg(tiles2d, grid->nz, per_sm);
-  }
-  a.zseg = std::min(zseg, grid->nz);
+  a.zseg = std::max(0, std::min(sc->zseg, grid->nz));
   return SWC_OK;
 }
 
@@ -693,31 +686,24 @@ int swc_rk_stage(const SwcGrid* grid, const SwcScheme* sc,
     return fail(SWC_ERR_UNSUPPORTED,
                 "transported scalars go through swc_rk_stage_ext");
   StageArgs a;
-  // Resident CTAs per SM of the plain stage kernel (its launch bounds):
-  // three for the inviscid single-precision MUSCL stage, two for the other
-  // single-precision ones, one in double precision.
-  const int per_sm = !sc || sc->dtype != SWC_F32 ? 1
-                     : (sc->interp == SWC_MUSCL && !sc->diffusion ? 3 : 2);
-  int st = stage_args(grid, sc, 5, per_sm, 16, uk,
-                      u0, uout, mode, c0, c1, dt, dtmin_out, a);
+  int st = stage_args(grid, sc, 5, uk, u0, uout, mode, c0, c1, dt, dtmin_out, a);
   if (st) return st;
   const int visc = sc->diffusion ? 1 : 0;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const int tile = sc->tile;
   int rc;
   if (sc->dtype == SWC_F32) {
     switch (sc->interp) {
-      case 0: rc = launch_stage_f32_s0(a, sc->riemann, visc, tile, s); break;
-      case 1: rc = launch_stage_f32_s1(a, sc->riemann, visc, tile, s); break;
-      case 2: rc = launch_stage_f32_s2(a, sc->riemann, visc, tile, s); break;
-      default: rc = launch_stage_f32_s3(a, sc->riemann, visc, tile, s); break;
+      case 0: rc = launch_stage_f32_s0(a, sc->riemann, visc, s); break;
+      case 1: rc = launch_stage_f32_s1(a, sc->riemann, visc, s); break;
+      case 2: rc = launch_stage_f32_s2(a, sc->riemann, visc, s); break;
+      default: rc = launch_stage_f32_s3(a, sc->riemann, visc, s); break;
     }
   } else {
     switch (sc->interp) {
-      case 0: rc = launch_stage_f64_s0(a, sc->riemann, visc, tile, s); break;
-      case 1: rc = launch_stage_f64_s1(a, sc->riemann, visc, tile, s); break;
-      case 2: rc = launch_stage_f64_s2(a, sc->riemann, visc, tile, s); break;
-      default: rc = launch_stage_f64_s3(a, sc->riemann, visc, tile, s); break;
+      case 0: rc = launch_stage_f64_s0(a, sc->riemann, visc, s); break;
+      case 1: rc = launch_stage_f64_s1(a, sc->riemann, visc, s); break;
+      case 2: rc = launch_stage_f64_s2(a, sc->riemann, visc, s); break;
+      default: rc = launch_stage_f64_s3(a, sc->riemann, visc, s); break;
     }
   }
   if (rc) return fail(rc, "stage launch failed: %s", cudaGetErrorString(cudaGetLastError()));
@@ -743,7 +729,7 @@ int swc_rk_stage_ext(const SwcGrid* grid, const SwcScheme* sc,
   }
   if ((e.p_ref == nullptr) != (e.rho_ref == nullptr))
     return fail(SWC_ERR_ARG, "p_ref and rho_ref go together");
-  bool any_face = false;
+  bool any_face = false, any_flux = false;
   for (int d = 0; d < 3; ++d)
     for (int sd = 0; sd < 2; ++sd) {
       if (e.nface[d][sd] < 0 || e.nface[d][sd] > SWC_MAX_OVERRIDES ||
@@ -766,6 +752,7 @@ int swc_rk_stage_ext(const SwcGrid* grid, const SwcScheme* sc,
             o.mode > SWC_FLUX_TOTAL)
           return fail(SWC_ERR_ARG, "bad flux override (var %d, type %d)", o.var,
                       o.mode);
+        any_flux = true;
       }
     }
   if (any_face && sc->diffusion)
@@ -773,27 +760,27 @@ int swc_rk_stage_ext(const SwcGrid* grid, const SwcScheme* sc,
                 "Face boundary conditions are not supported with diffusion "
                 "enabled at this time.");
   StageArgs a;
-  int st = stage_args(grid, sc, 5 + ns, 1,
-                      sc && sc->dtype == SWC_F64 ? 8 : 16, uk, u0, uout, mode,
-                      c0, c1, dt, dtmin_out, a);
+  int st = stage_args(grid, sc, 5 + ns, uk, u0, uout, mode, c0, c1, dt,
+                      dtmin_out, a);
   if (st) return st;
   const int visc = sc->diffusion ? 1 : 0;
   const int help = e.p_ref ? 1 : 0;
+  const int ov = any_face || any_flux ? 1 : 0;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   int rc;
   if (sc->dtype == SWC_F32) {
     switch (sc->interp) {
-      case 0: rc = launch_stage_ext_f32_s0(a, e, sc->riemann, visc, ns, help, s); break;
-      case 1: rc = launch_stage_ext_f32_s1(a, e, sc->riemann, visc, ns, help, s); break;
-      case 2: rc = launch_stage_ext_f32_s2(a, e, sc->riemann, visc, ns, help, s); break;
-      default: rc = launch_stage_ext_f32_s3(a, e, sc->riemann, visc, ns, help, s); break;
+      case 0: rc = launch_stage_ext_f32_s0(a, e, sc->riemann, visc, ns, help, ov, s); break;
+      case 1: rc = launch_stage_ext_f32_s1(a, e, sc->riemann, visc, ns, help, ov, s); break;
+      case 2: rc = launch_stage_ext_f32_s2(a, e, sc->riemann, visc, ns, help, ov, s); break;
+      default: rc = launch_stage_ext_f32_s3(a, e, sc->riemann, visc, ns, help, ov, s); break;
     }
   } else {
     switch (sc->interp) {
-      case 0: rc = launch_stage_ext_f64_s0(a, e, sc->riemann, visc, ns, help, s); break;
-      case 1: rc = launch_stage_ext_f64_s1(a, e, sc->riemann, visc, ns, help, s); break;
-      case 2: rc = launch_stage_ext_f64_s2(a, e, sc->riemann, visc, ns, help, s); break;
-      default: rc = launch_stage_ext_f64_s3(a, e, sc->riemann, visc, ns, help, s); break;
+      case 0: rc = launch_stage_ext_f64_s0(a, e, sc->riemann, visc, ns, help, ov, s); break;
+      case 1: rc = launch_stage_ext_f64_s1(a, e, sc->riemann, visc, ns, help, ov, s); break;
+      case 2: rc = launch_stage_ext_f64_s2(a, e, sc->riemann, visc, ns, help, ov, s); break;
+      default: rc = launch_stage_ext_f64_s3(a, e, sc->riemann, visc, ns, help, ov, s); break;
     }
   }
   if (rc) return fail(rc, "stage launch failed: %s", cudaGetErrorString(cudaGetLastError()));

@@ -24,14 +24,13 @@ struct NvtxRange {
 // negative SWC status. Defined in swc_stage_inst.cu, compiled once per pair.
 #define SWC_DECL_STAGE(SUFFIX)                                               \
   int launch_stage_##SUFFIX(const StageArgs& a, int riemann, int visc,       \
-                            int tile, cudaStream_t st);                      \
+                            cudaStream_t st);                                \
   int launch_stage_batch_##SUFFIX(const StageBatch& b, int nblocks,          \
                                   int riemann, int visc, int tile,           \
                                   cudaStream_t st);                          \
   int launch_stage_ext_##SUFFIX(const StageArgs& a, const SwcStageExt& e,   \
                                 int riemann, int visc, int ns, int help,     \
-                                cudaStream_t st);                            \
-  size_t stage_smem_##SUFFIX(int visc, int tile);                          \
+                                int overrides, cudaStream_t st);             \
   size_t stage_batch_smem_##SUFFIX(int visc, int tile);
 SWC_DECL_STAGE(f32_s0)
 SWC_DECL_STAGE(f32_s1)
@@ -52,6 +51,10 @@ inline int stage_halo_needed(int scheme, int visc) {
     default: return visc ? Geom<3, true>::NEED : Geom<3, false>::NEED;
   }
 }
+
+// z planes per CTA for `tiles2d` (y, x) tiles and `per_sm` resident CTAs per
+// SM.
+int auto_zseg(long long tiles2d, int nz, int per_sm);
 
 // Counts kernel launches issued by this library (thread-local).
 void note_launch(int n = 1);

@@ -805,13 +805,43 @@ __global__ void __launch_bounds__(TY* TX, (stage_min_blocks<T, SCHEME, VISC>()))
                                                blockIdx.y * TX, blockIdx.z);
 }
 
-// Extended stage: NS transported scalars, HELP reference states, face and
-// flux overrides on the grid boundary (one CTA per SM: the ring is larger).
+// Tile and resident CTAs per SM of an extended stage, whose ring is larger by
+// the scalars and p_dyn: the first of these that shared memory holds (228 KB
+// per SM, 1 KB of it reserved per CTA). Two CTAs hide each other's barriers
+// and four to six more warps hide latency: with one 16 x 16 CTA (8 warps) the
+// issue slots were 27 % busy.
+//   single precision: 2 x (16 x 16), 2 x (16 x 12), 1 x (16 x 24)
+//   double precision: 1 x (16 x 16), 1 x (16 x 12), 1 x (8 x 16)
+// EXT (face and flux overrides, few and small in practice) keeps one CTA and
+// its registers.
+struct ExtTile {
+  int ty, tx, ctas;
+};
+template <typename T, int SCHEME, bool VISC, int NS, bool HELP, bool EXT>
+constexpr ExtTile ext_tile() {
+  constexpr size_t kSm = 228 * 1024, kCta = 1024 + 512;  // + static shared
+  constexpr size_t s16 = Layout<T, SCHEME, VISC, 16, 16, NS, HELP>::SMEM + kCta;
+  constexpr size_t s12 = Layout<T, SCHEME, VISC, 16, 12, NS, HELP>::SMEM + kCta;
+  constexpr size_t s24 = Layout<T, SCHEME, VISC, 16, 24, NS, HELP>::SMEM + kCta;
+  if (sizeof(T) == 4) {
+    if (EXT) return {16, 16, 1};
+    if (2 * s16 <= kSm) return {16, 16, 2};
+    if (2 * s12 <= kSm) return {16, 12, 2};
+    if (s24 <= kSm) return {16, 24, 1};
+    return {16, 16, 1};
+  }
+  if (s16 <= kSm) return {16, 16, 1};
+  if (s12 <= kSm) return {16, 12, 1};
+  return {8, 16, 1};
+}
+
+// Extended stage: NS transported scalars, HELP reference states, EXT face and
+// flux overrides on the grid boundary.
 template <typename T, int SCHEME, int RIEMANN, bool VISC, int TY, int TX,
-          int NS, bool HELP>
-__global__ void __launch_bounds__(TY* TX, 1)
+          int CTAS, int NS, bool HELP, bool EXT>
+__global__ void __launch_bounds__(TY* TX, CTAS)
     stage_kernel_ext(const StageArgs a, const SwcStageExt e) {
-  stage_body<T, SCHEME, RIEMANN, VISC, TY, TX, NS, HELP, true>(
+  stage_body<T, SCHEME, RIEMANN, VISC, TY, TX, NS, HELP, EXT>(
       a, &e, blockIdx.x * TY, blockIdx.y * TX, blockIdx.z);
 }
 

@@ -7,19 +7,29 @@
 #error "SWC_T must be defined"
 #endif
 
-#ifndef SWC_MULTI_TILE
-#define SWC_MULTI_TILE 0
-#endif
-
 #define SWC_CAT2(a, b) a##b
 #define SWC_CAT(a, b) SWC_CAT2(a, b)
 
 namespace swc {
 namespace {
 
-// Tile shapes (TY along y, TX along x); 256 threads each.
-template <typename T, int RM, bool V, int TY, int TX>
-int launch_tile(const StageArgs& a, cudaStream_t st) {
+// `a` with the z segment filled in where the caller left it to the library.
+StageArgs with_zseg(const StageArgs& a, int ty, int tx, int per_sm) {
+  StageArgs b = a;
+  if (b.zseg <= 0)
+    b.zseg = auto_zseg((long long)((a.ny + ty - 1) / ty) *
+                           ((a.nx + tx - 1) / tx), a.nz, per_sm);
+  b.zseg = b.zseg < a.nz ? b.zseg : a.nz;
+  return b;
+}
+dim3 stage_grid(const StageArgs& a, int ty, int tx) {
+  return dim3((a.ny + ty - 1) / ty, (a.nx + tx - 1) / tx,
+              (a.nz + a.zseg - 1) / a.zseg);
+}
+
+template <typename T, int RM, bool V>
+int launch_rm(const StageArgs& a, cudaStream_t st) {
+  constexpr int TY = 16, TX = 16;
   using Lay = Layout<T, SWC_SCHEME, V, TY, TX>;
   auto kern = stage_kernel<T, SWC_SCHEME, RM, V, TY, TX>;
   // Set once per process (before any graph capture: the first launch of a
@@ -32,26 +42,12 @@ int launch_tile(const StageArgs& a, cudaStream_t st) {
     if (e != cudaSuccess) return SWC_ERR_LAUNCH;
     attr_set = 1;
   }
-  dim3 grid((a.ny + TY - 1) / TY, (a.nx + TX - 1) / TX,
-            (a.nz + a.zseg - 1) / a.zseg);
-  kern<<<grid, TY * TX, Lay::SMEM, st>>>(a);
+  const StageArgs b =
+      with_zseg(a, TY, TX, stage_min_blocks<T, SWC_SCHEME, V>());
+  kern<<<stage_grid(b, TY, TX), TY * TX, Lay::SMEM, st>>>(b);
   note_launch();
   e = cudaGetLastError();
   return e == cudaSuccess ? SWC_OK : SWC_ERR_LAUNCH;
-}
-
-template <typename T, int RM, bool V>
-int launch_rm(const StageArgs& a, int tile, cudaStream_t st) {
-#if SWC_MULTI_TILE
-  switch (tile) {
-    case 1: return launch_tile<T, RM, V, 16, 16>(a, st);
-    case 2: return launch_tile<T, RM, V, 8, 32>(a, st);
-    default: return launch_tile<T, RM, V, 32, 8>(a, st);
-  }
-#else
-  (void)tile;
-  return launch_tile<T, RM, V, 16, 16>(a, st);
-#endif
 }
 
 // Batched launch of `nblocks` CTAs over the members of `b`. Tiles: 1 = 16x16
@@ -81,13 +77,15 @@ int launch_batch_rm(const StageBatch& b, int nblocks, int tile,
   return launch_batch_tile<T, RM, V, 16, 16>(b, nblocks, st);
 }
 
-// Extended stage (scalars, helper states, face/flux overrides): 16x16 tiles
-// in f32, 8x16 in f64 so that the larger ring fits in shared memory.
-template <typename T, int RM, bool V, int NS, bool HELP>
+// Extended stage (scalars, helper states, face/flux overrides); the tile is
+// ext_tile's.
+template <typename T, int RM, bool V, int NS, bool HELP, bool EXT>
 int launch_ext_v(const StageArgs& a, const SwcStageExt& e, cudaStream_t st) {
-  constexpr int TY = sizeof(T) == 4 ? 16 : 8, TX = 16;
+  constexpr ExtTile kT = ext_tile<T, SWC_SCHEME, V, NS, HELP, EXT>();
+  constexpr int TY = kT.ty, TX = kT.tx;
   using Lay = Layout<T, SWC_SCHEME, V, TY, TX, NS, HELP>;
-  auto kern = stage_kernel_ext<T, SWC_SCHEME, RM, V, TY, TX, NS, HELP>;
+  auto kern = stage_kernel_ext<T, SWC_SCHEME, RM, V, TY, TX, kT.ctas, NS, HELP,
+                               EXT>;
   static int attr_set = 0;
   cudaError_t err;
   if (!attr_set) {
@@ -96,53 +94,42 @@ int launch_ext_v(const StageArgs& a, const SwcStageExt& e, cudaStream_t st) {
     if (err != cudaSuccess) return SWC_ERR_LAUNCH;
     attr_set = 1;
   }
-  dim3 grid((a.ny + TY - 1) / TY, (a.nx + TX - 1) / TX,
-            (a.nz + a.zseg - 1) / a.zseg);
-  kern<<<grid, TY * TX, Lay::SMEM, st>>>(a, e);
+  const StageArgs b = with_zseg(a, TY, TX, kT.ctas);
+  kern<<<stage_grid(b, TY, TX), TY * TX, Lay::SMEM, st>>>(b, e);
   note_launch();
   err = cudaGetLastError();
   return err == cudaSuccess ? SWC_OK : SWC_ERR_LAUNCH;
 }
 
-template <typename T, int RM, bool V>
+template <typename T, int RM, bool V, bool EXT>
 int launch_ext_rm(const StageArgs& a, const SwcStageExt& e, int ns, bool help,
                   cudaStream_t st) {
   switch (ns * 2 + (help ? 1 : 0)) {
-    case 0: return launch_ext_v<T, RM, V, 0, false>(a, e, st);
-    case 1: return launch_ext_v<T, RM, V, 0, true>(a, e, st);
-    case 2: return launch_ext_v<T, RM, V, 1, false>(a, e, st);
-    case 3: return launch_ext_v<T, RM, V, 1, true>(a, e, st);
-    case 4: return launch_ext_v<T, RM, V, 2, false>(a, e, st);
-    case 5: return launch_ext_v<T, RM, V, 2, true>(a, e, st);
-    case 6: return launch_ext_v<T, RM, V, 3, false>(a, e, st);
-    default: return launch_ext_v<T, RM, V, 3, true>(a, e, st);
+    case 0: return launch_ext_v<T, RM, V, 0, false, EXT>(a, e, st);
+    case 1: return launch_ext_v<T, RM, V, 0, true, EXT>(a, e, st);
+    case 2: return launch_ext_v<T, RM, V, 1, false, EXT>(a, e, st);
+    case 3: return launch_ext_v<T, RM, V, 1, true, EXT>(a, e, st);
+    case 4: return launch_ext_v<T, RM, V, 2, false, EXT>(a, e, st);
+    case 5: return launch_ext_v<T, RM, V, 2, true, EXT>(a, e, st);
+    case 6: return launch_ext_v<T, RM, V, 3, false, EXT>(a, e, st);
+    default: return launch_ext_v<T, RM, V, 3, true, EXT>(a, e, st);
   }
 }
-
-template <typename T, bool V>
-size_t smem_tile(int tile) {
-#if SWC_MULTI_TILE
-  switch (tile) {
-    case 1: return Layout<T, SWC_SCHEME, V, 16, 16>::SMEM;
-    case 2: return Layout<T, SWC_SCHEME, V, 8, 32>::SMEM;
-    default: return Layout<T, SWC_SCHEME, V, 32, 8>::SMEM;
-  }
-#else
-  (void)tile;
-  return Layout<T, SWC_SCHEME, V, 16, 16>::SMEM;
-#endif
+template <typename T, int RM, bool V>
+int launch_ext_rm(const StageArgs& a, const SwcStageExt& e, int ns, bool help,
+                  bool overrides, cudaStream_t st) {
+  return overrides ? launch_ext_rm<T, RM, V, true>(a, e, ns, help, st)
+                   : launch_ext_rm<T, RM, V, false>(a, e, ns, help, st);
 }
 
 }  // namespace
 
 int SWC_CAT(launch_stage_, SWC_SUFFIX)(const StageArgs& a, int riemann,
-                                       int visc, int tile, cudaStream_t st) {
+                                       int visc, cudaStream_t st) {
   using T = SWC_T;
   if (riemann == SWC_HLL)
-    return visc ? launch_rm<T, 0, true>(a, tile, st)
-                : launch_rm<T, 0, false>(a, tile, st);
-  return visc ? launch_rm<T, 1, true>(a, tile, st)
-              : launch_rm<T, 1, false>(a, tile, st);
+    return visc ? launch_rm<T, 0, true>(a, st) : launch_rm<T, 0, false>(a, st);
+  return visc ? launch_rm<T, 1, true>(a, st) : launch_rm<T, 1, false>(a, st);
 }
 
 int SWC_CAT(launch_stage_batch_, SWC_SUFFIX)(const StageBatch& b, int nblocks,
@@ -159,14 +146,14 @@ int SWC_CAT(launch_stage_batch_, SWC_SUFFIX)(const StageBatch& b, int nblocks,
 int SWC_CAT(launch_stage_ext_, SWC_SUFFIX)(const StageArgs& a,
                                            const SwcStageExt& e, int riemann,
                                            int visc, int ns, int help,
-                                           cudaStream_t st) {
+                                           int overrides, cudaStream_t st) {
   using T = SWC_T;
-  const bool hp = help != 0;
+  const bool hp = help != 0, ov = overrides != 0;
   if (riemann == SWC_HLL)
-    return visc ? launch_ext_rm<T, 0, true>(a, e, ns, hp, st)
-                : launch_ext_rm<T, 0, false>(a, e, ns, hp, st);
-  return visc ? launch_ext_rm<T, 1, true>(a, e, ns, hp, st)
-              : launch_ext_rm<T, 1, false>(a, e, ns, hp, st);
+    return visc ? launch_ext_rm<T, 0, true>(a, e, ns, hp, ov, st)
+                : launch_ext_rm<T, 0, false>(a, e, ns, hp, ov, st);
+  return visc ? launch_ext_rm<T, 1, true>(a, e, ns, hp, ov, st)
+              : launch_ext_rm<T, 1, false>(a, e, ns, hp, ov, st);
 }
 
 size_t SWC_CAT(stage_batch_smem_, SWC_SUFFIX)(int visc, int tile) {
@@ -176,11 +163,6 @@ size_t SWC_CAT(stage_batch_smem_, SWC_SUFFIX)(int visc, int tile) {
                 : Layout<T, SWC_SCHEME, false, 8, 32>::SMEM;
   return visc ? Layout<T, SWC_SCHEME, true, 16, 16>::SMEM
               : Layout<T, SWC_SCHEME, false, 16, 16>::SMEM;
-}
-
-size_t SWC_CAT(stage_smem_, SWC_SUFFIX)(int visc, int tile) {
-  using T = SWC_T;
-  return visc ? smem_tile<T, true>(tile) : smem_tile<T, false>(tile);
 }
 
 }  // namespace swc
