@@ -317,20 +317,22 @@ int launch_stage_group(const SwcScheme* sc, const StageBatch& b, int tile,
   if (b.n == 0) return SWC_OK;
   const int visc = sc->diffusion ? 1 : 0;
   const int nblocks = b.pre[b.n];
+  int pe = 0;
+  for (int i = 0; i < b.n; ++i) pe |= b.m[i].has_pe;
   int rc;
   if (sc->dtype == SWC_F32) {
     switch (sc->interp) {
-      case 0: rc = launch_stage_batch_f32_s0(b, nblocks, sc->riemann, visc, tile, s); break;
-      case 1: rc = launch_stage_batch_f32_s1(b, nblocks, sc->riemann, visc, tile, s); break;
-      case 2: rc = launch_stage_batch_f32_s2(b, nblocks, sc->riemann, visc, tile, s); break;
-      default: rc = launch_stage_batch_f32_s3(b, nblocks, sc->riemann, visc, tile, s); break;
+      case 0: rc = launch_stage_batch_f32_s0(b, nblocks, sc->riemann, visc, tile, pe, s); break;
+      case 1: rc = launch_stage_batch_f32_s1(b, nblocks, sc->riemann, visc, tile, pe, s); break;
+      case 2: rc = launch_stage_batch_f32_s2(b, nblocks, sc->riemann, visc, tile, pe, s); break;
+      default: rc = launch_stage_batch_f32_s3(b, nblocks, sc->riemann, visc, tile, pe, s); break;
     }
   } else {
     switch (sc->interp) {
-      case 0: rc = launch_stage_batch_f64_s0(b, nblocks, sc->riemann, visc, tile, s); break;
-      case 1: rc = launch_stage_batch_f64_s1(b, nblocks, sc->riemann, visc, tile, s); break;
-      case 2: rc = launch_stage_batch_f64_s2(b, nblocks, sc->riemann, visc, tile, s); break;
-      default: rc = launch_stage_batch_f64_s3(b, nblocks, sc->riemann, visc, tile, s); break;
+      case 0: rc = launch_stage_batch_f64_s0(b, nblocks, sc->riemann, visc, tile, pe, s); break;
+      case 1: rc = launch_stage_batch_f64_s1(b, nblocks, sc->riemann, visc, tile, pe, s); break;
+      case 2: rc = launch_stage_batch_f64_s2(b, nblocks, sc->riemann, visc, tile, pe, s); break;
+      default: rc = launch_stage_batch_f64_s3(b, nblocks, sc->riemann, visc, tile, pe, s); break;
     }
   }
   if (rc)

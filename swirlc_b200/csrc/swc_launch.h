@@ -26,7 +26,7 @@ struct NvtxRange {
   int launch_stage_##SUFFIX(const StageArgs& a, int riemann, int visc,       \
                             cudaStream_t st);                                \
   int launch_stage_batch_##SUFFIX(const StageBatch& b, int nblocks,          \
-                                  int riemann, int visc, int tile,           \
+                                  int riemann, int visc, int tile, int pe,   \
                                   cudaStream_t st);                          \
   int launch_stage_ext_##SUFFIX(const StageArgs& a, const SwcStageExt& e,   \
                                 int riemann, int visc, int ns, int help,     \

@@ -27,11 +27,11 @@ dim3 stage_grid(const StageArgs& a, int ty, int tx) {
               (a.nz + a.zseg - 1) / a.zseg);
 }
 
-template <typename T, int RM, bool V>
-int launch_rm(const StageArgs& a, cudaStream_t st) {
+template <typename T, int RM, bool V, bool PE>
+int launch_plain(const StageArgs& a, cudaStream_t st) {
   constexpr int TY = 16, TX = 16;
   using Lay = Layout<T, SWC_SCHEME, V, TY, TX>;
-  auto kern = stage_kernel<T, SWC_SCHEME, RM, V, TY, TX>;
+  auto kern = stage_kernel<T, SWC_SCHEME, RM, V, TY, TX, PE>;
   // Set once per process (before any graph capture: the first launch of a
   // variant is always eager).
   static int attr_set = 0;
@@ -50,12 +50,18 @@ int launch_rm(const StageArgs& a, cudaStream_t st) {
   return e == cudaSuccess ? SWC_OK : SWC_ERR_LAUNCH;
 }
 
+template <typename T, int RM, bool V>
+int launch_rm(const StageArgs& a, cudaStream_t st) {
+  return a.has_pe ? launch_plain<T, RM, V, true>(a, st)
+                  : launch_plain<T, RM, V, false>(a, st);
+}
+
 // Batched launch of `nblocks` CTAs over the members of `b`. Tiles: 1 = 16x16
 // (y x x), 2 = 8x32 for members with ny <= 8.
-template <typename T, int RM, bool V, int TY, int TX>
+template <typename T, int RM, bool V, int TY, int TX, bool PE>
 int launch_batch_tile(const StageBatch& b, int nblocks, cudaStream_t st) {
   using Lay = Layout<T, SWC_SCHEME, V, TY, TX>;
-  auto kern = stage_batch_kernel<T, SWC_SCHEME, RM, V, TY, TX>;
+  auto kern = stage_batch_kernel<T, SWC_SCHEME, RM, V, TY, TX, PE>;
   static int attr_set = 0;
   cudaError_t e;
   if (!attr_set) {
@@ -71,10 +77,13 @@ int launch_batch_tile(const StageBatch& b, int nblocks, cudaStream_t st) {
 }
 
 template <typename T, int RM, bool V>
-int launch_batch_rm(const StageBatch& b, int nblocks, int tile,
+int launch_batch_rm(const StageBatch& b, int nblocks, int tile, int pe,
                     cudaStream_t st) {
-  if (tile == 2) return launch_batch_tile<T, RM, V, 8, 32>(b, nblocks, st);
-  return launch_batch_tile<T, RM, V, 16, 16>(b, nblocks, st);
+  if (tile == 2)
+    return pe ? launch_batch_tile<T, RM, V, 8, 32, true>(b, nblocks, st)
+              : launch_batch_tile<T, RM, V, 8, 32, false>(b, nblocks, st);
+  return pe ? launch_batch_tile<T, RM, V, 16, 16, true>(b, nblocks, st)
+            : launch_batch_tile<T, RM, V, 16, 16, false>(b, nblocks, st);
 }
 
 // Extended stage (scalars, helper states, face/flux overrides); the tile is
@@ -134,13 +143,13 @@ int SWC_CAT(launch_stage_, SWC_SUFFIX)(const StageArgs& a, int riemann,
 
 int SWC_CAT(launch_stage_batch_, SWC_SUFFIX)(const StageBatch& b, int nblocks,
                                              int riemann, int visc, int tile,
-                                             cudaStream_t st) {
+                                             int pe, cudaStream_t st) {
   using T = SWC_T;
   if (riemann == SWC_HLL)
-    return visc ? launch_batch_rm<T, 0, true>(b, nblocks, tile, st)
-                : launch_batch_rm<T, 0, false>(b, nblocks, tile, st);
-  return visc ? launch_batch_rm<T, 1, true>(b, nblocks, tile, st)
-              : launch_batch_rm<T, 1, false>(b, nblocks, tile, st);
+    return visc ? launch_batch_rm<T, 0, true>(b, nblocks, tile, pe, st)
+                : launch_batch_rm<T, 0, false>(b, nblocks, tile, pe, st);
+  return visc ? launch_batch_rm<T, 1, true>(b, nblocks, tile, pe, st)
+              : launch_batch_rm<T, 1, false>(b, nblocks, tile, pe, st);
 }
 
 int SWC_CAT(launch_stage_ext_, SWC_SUFFIX)(const StageArgs& a,
