@@ -450,18 +450,37 @@ extern "C" int swc_batch_step(const SwcScheme* sc, int32_t order,
                           batch_smem(sc, 2));
     plans[i].tile = members[i].tile ? members[i].tile : 1;
   }
-  // z planes per CTA for the members that leave it to us: the largest of
-  // 64, 32, 16, 8 that still gives about four waves of CTAs (2 per SM on
-  // 148 SMs) over the whole batch; longer segments amortise the ring warm-up.
-  int zauto = 8;
-  for (int z : {64, 32, 16, 8}) {
-    long long total = 0;
+  // z planes per CTA for the members that leave it to us: the one of 64, 32 ..
+  // 1 with the least time over the whole batch. A CTA takes zseg + 1 planes'
+  // time (auto_zseg); k of them resident on an SM take (k + 1) / 2 of one's.
+  // A launch takes that of its longest CTA at the occupancy it reaches, or the
+  // sum over all CTAs at full occupancy and half of the longest CTA, while
+  // the last ones drain. Long segments amortise the ring warm-up; a batch of
+  // few small grids needs short ones to reach every SM.
+  const int per_sm = sc->dtype == SWC_F32 ? 2 : 1;
+  int zauto = 64;
+  double least = -1.0;
+  for (int z : {64, 32, 16, 8, 4, 2, 1}) {
+    long long total = 0, planes = 0;
+    int longest = 0;
     for (const Plan& p : plans) {
       const int nz = p.m->grid.nz;
       const int zs = p.m->zseg ? std::min(p.m->zseg, nz) : std::min(z, nz);
-      total += tiles2d(p.m->grid, p.tile) * ((nz + zs - 1) / zs);
+      const long long nseg = (nz + zs - 1) / zs;
+      total += tiles2d(p.m->grid, p.tile) * nseg;
+      planes += tiles2d(p.m->grid, p.tile) * (nz + nseg);
+      longest = std::max(longest, zs + 1);
     }
-    if (total >= 4LL * 2 * 148) { zauto = z; break; }
+    const long long sms = sm_count();
+    const double k = (double)std::min<long long>((total + sms - 1) / sms, per_sm);
+    const double one = longest * (k + 1) / 2;
+    const double all = (double)planes / sms * (per_sm + 1) / (2 * per_sm) +
+                       0.5 * longest;
+    const double cost = std::max(one, all);
+    if (least < 0 || cost < least) {
+      least = cost;
+      zauto = z;
+    }
   }
   for (Plan& p : plans) {
     const int nz = p.m->grid.nz;

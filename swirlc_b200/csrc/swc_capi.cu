@@ -419,7 +419,7 @@ __global__ void viscous_terms_kernel(const ViscArgs a) {
 }
 
 // SMs of the current device (queried once per device).
-static int sm_count() {
+int sm_count() {
   static int cached[64] = {0};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
@@ -434,22 +434,32 @@ static int sm_count() {
 
 // Automatic z segment of the stage kernel for `tiles2d` (y, x) tiles and
 // `per_sm` resident CTAs per SM. A CTA's time is about (zseg + 1) planes
-// (the extra plane: warm-up and the z face below the segment), and the
-// launch takes ceil(CTAs / slots) rounds of them, so the segment count that
-// minimises rounds x (zseg + 1) is taken: at 256^3 that is 8 segments of 32
-// planes (7 rounds of 2048 CTAs on 296 slots) rather than a last round that
-// leaves most SMs idle.
+// (the extra plane: warm-up and the z face below the segment). One CTA alone
+// on an SM takes 4.6 us per plane (WENO5, single precision) and every further
+// resident one adds half of that, so k of them cost (k + 1) / 2; CTAs are
+// dealt out evenly, `per_sm` at a time, and the shorter CTAs of the last
+// segment count only where they need a place of their own. In units of half a
+// plane this reproduces measured steps of 256 x 8 x 8 to 128 x 96 x 100 cells
+// within 15 % for every segment length.
+// Grids of up to a CTA per SM take one plane per CTA: a step of 256 x 8 x 8
+// cells takes 80 us at four planes and 41 us at one, 32^3 76 and 43 us;
+// 61 x 47 x 33 90 us at four, 76 at three, 86 at one (three CTAs on an SM).
+// At 256^3 it is 8 segments of 32 planes.
 int auto_zseg(long long tiles2d, int nz, int per_sm) {
-  const long long slots = (long long)sm_count() * per_sm;
+  const long long sms = sm_count();
+  auto units = [&](long long ctas) -> long long {
+    const long long m = (ctas + sms - 1) / sms, r = m % per_sm;
+    return m / per_sm * (per_sm + 1) + (r ? r + 1 : 0);
+  };
   long long best_cost = -1;
   int best = nz;
   for (int nseg = 1; nseg <= nz; ++nseg) {
     const int zs = (nz + nseg - 1) / nseg;
     if (nseg > 1 && zs == (nz + nseg - 2) / (nseg - 1)) continue;  // same zseg
-    if (zs < 4 && nseg > 1) break;
-    const long long segs = (nz + zs - 1) / zs;
-    const long long rounds = (tiles2d * segs + slots - 1) / slots;
-    const long long cost = rounds * (zs + 1);
+    const long long full = nz / zs, rem = nz % zs;
+    const long long u = units(tiles2d * full);
+    long long cost = u * (zs + 1);
+    if (rem) cost += (units(tiles2d * (full + 1)) - u) * (rem + 1);
     if (best_cost < 0 || cost < best_cost) {
       best_cost = cost;
       best = zs;

@@ -52,6 +52,9 @@ inline int stage_halo_needed(int scheme, int visc) {
   }
 }
 
+// SMs of the current device (queried once per device).
+int sm_count();
+
 // z planes per CTA for `tiles2d` (y, x) tiles and `per_sm` resident CTAs per
 // SM.
 int auto_zseg(long long tiles2d, int nz, int per_sm);
