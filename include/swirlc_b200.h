@@ -126,6 +126,15 @@ int swc_halo_fill(const SwcGrid* grid, int32_t dtype, int32_t nfields,
                   void* const* fields, const SwcFieldBC* bcs,
                   int32_t rho_index, void* stream);
 
+/* Copies of `src` with their halos filled, in `dst`; `src` stays as it is (its
+ * halos are not read on sides with a boundary condition). `clear`, when not
+ * NULL, holds one more array per field whose halo cells are set to 0 (its
+ * interior may be, too). No dst or clear array may be a src array. */
+int swc_halo_copy(const SwcGrid* grid, int32_t dtype, int32_t nfields,
+                  const void* const* src, void* const* dst,
+                  void* const* clear, const SwcFieldBC* bcs,
+                  int32_t rho_index, void* stream);
+
 /* One fused pass: RHS of the conserved state `uk` (halos already filled)
  * followed by the stage combination selected by `mode`. `u0` may be NULL
  * for SWC_OUT_RHS / SWC_OUT_EULER; `uout` may alias `u0` (pointwise) but
@@ -202,6 +211,21 @@ int swc_rk_stage_ext(const SwcGrid* grid, const SwcScheme* scheme,
 int swc_rk_step(const SwcGrid* grid, const SwcScheme* scheme,
                 const SwcFieldBC* bcs, int32_t order, void* const* u,
                 void* const* work, SwcClock* clock_dev, void* stream);
+
+/* Functional forms on 5 + scheme->nscalars fields, which stay as they are.
+ * `ext` NULL: the plain stage, else swc_rk_stage_ext's. swc_rhs writes the time
+ * derivative of every cell, zero in the halos (get_rhs_fn's rhs,
+ * compressible_navier_stokes.py:68-268); `work` holds one buffer per field.
+ * swc_rk_step_out writes the state after one step of *dt (a device double),
+ * halos filled (rk3.py:87-120, rk2.py:69-86); `work` holds two per field. */
+int swc_rhs(const SwcGrid* grid, const SwcScheme* scheme,
+            const SwcFieldBC* bcs, const SwcStageExt* ext,
+            const void* const* u, void* const* out, void* const* work,
+            void* stream);
+int swc_rk_step_out(const SwcGrid* grid, const SwcScheme* scheme,
+                    const SwcFieldBC* bcs, const SwcStageExt* ext,
+                    int32_t order, const void* const* u, void* const* out,
+                    void* const* work, const double* dt, void* stream);
 
 /* Size of the built-in work space of swc_rk_step_noalloc (64 MiB). */
 #define SWC_NOALLOC_MAX_BYTES (64ll << 20)

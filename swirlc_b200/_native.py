@@ -8,6 +8,7 @@ compute entry point raises.
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 import threading
 from typing import Optional, Sequence
@@ -44,7 +45,7 @@ EXPORTED = (
     'swc_rk_step',
     'swc_rk_step_noalloc', 'swc_batch_step', 'swc_rk_stage_ext',
     'swc_rk_stage_vjp',
-    'swc_rk_step_vjp',
+    'swc_rk_step_vjp', 'swc_halo_copy', 'swc_rhs', 'swc_rk_step_out',
 )
 
 # Built-in work space of swc_rk_step_noalloc (SWC_NOALLOC_MAX_BYTES).
@@ -115,6 +116,7 @@ class SwcBatchMember(ctypes.Structure):
 
 
 _lib: Optional[ctypes.CDLL] = None
+_cuda_seen = False
 _lock = threading.Lock()
 
 
@@ -124,9 +126,14 @@ def lib_path() -> str:
 
 def load(require_cuda: bool = True) -> ctypes.CDLL:
   """Loads the library; raises if it is missing (no fallback path exists)."""
-  global _lib
+  global _lib, _cuda_seen
+  # Once a device was seen the check is not repeated: it takes 8 us, and a
+  # functional step calls this several times.
+  if _lib is not None and (_cuda_seen or not require_cuda):
+    return _lib
   if require_cuda and not torch.cuda.is_available():
     raise RuntimeError('swirlc_b200 needs a CUDA device; none is visible.')
+  _cuda_seen = _cuda_seen or require_cuda
   with _lock:
     if _lib is None:
       if not os.path.exists(_LIB_PATH):
@@ -180,6 +187,17 @@ def load(require_cuda: bool = True) -> ctypes.CDLL:
                                       pp, pp, pp, vp, pp, vp]
       lib.swc_batch_step.argtypes = [ctypes.POINTER(SwcScheme), i32, i32,
                                      ctypes.POINTER(SwcBatchMember), vp]
+      lib.swc_halo_copy.argtypes = [ctypes.POINTER(SwcGrid), i32, i32, pp, pp,
+                                    pp, ctypes.POINTER(SwcFieldBC), i32, vp]
+      lib.swc_rhs.argtypes = [ctypes.POINTER(SwcGrid),
+                              ctypes.POINTER(SwcScheme),
+                              ctypes.POINTER(SwcFieldBC),
+                              ctypes.POINTER(SwcStageExt), pp, pp, pp, vp]
+      lib.swc_rk_step_out.argtypes = [ctypes.POINTER(SwcGrid),
+                                      ctypes.POINTER(SwcScheme),
+                                      ctypes.POINTER(SwcFieldBC),
+                                      ctypes.POINTER(SwcStageExt), i32, pp, pp,
+                                      pp, vp, vp]
       lib.swc_rk_step_noalloc.argtypes = [ctypes.POINTER(SwcGrid),
                                           ctypes.POINTER(SwcScheme),
                                           ctypes.POINTER(SwcFieldBC), i32, pp,
@@ -220,23 +238,24 @@ def launch_count() -> int:
 
 
 def stream_ptr(stream: Optional[torch.cuda.Stream] = None) -> int:
-  s = stream if stream is not None else torch.cuda.current_stream()
-  return int(s.cuda_stream)
+  if stream is None:
+    # torch.cuda.current_stream() without the Stream object (4 us a call).
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+  return int(stream.cuda_stream)
+
+
+@functools.lru_cache(maxsize=None)
+def _array_type(n: int):
+  return ctypes.c_void_p * n
 
 
 def ptr_array(tensors: Sequence[Optional[torch.Tensor]]):
-  arr = (ctypes.c_void_p * max(1, len(tensors)))()
-  for i, t in enumerate(tensors):
-    arr[i] = None if t is None else t.data_ptr()
-  return arr
+  return addr_array([None if t is None else t.data_ptr() for t in tensors])
 
 
 def addr_array(addrs: Sequence[Optional[int]]):
   """A void* array from raw device addresses (None for NULL)."""
-  arr = (ctypes.c_void_p * max(1, len(addrs)))()
-  for i, a in enumerate(addrs):
-    arr[i] = a
-  return arr
+  return _array_type(max(1, len(addrs)))(*addrs)
 
 
 def dtype_code(dtype: torch.dtype) -> int:

@@ -77,20 +77,49 @@ __global__ void halo_kernel(const HaloArgs a) {
     halo_elem<T>(a, t);
 }
 
+// What a one-pass halo fill does to the device clock beside its own work, so
+// that a step needs no launches for it: the fill before the first stage
+// starts the step, the fill before the last one ends it (no kernel of the
+// step reads or writes t or the step count in between).
+enum ClockTick { kTickNone, kTickBegin, kTickEnd };
+__device__ __forceinline__ void clock_tick(SwcClock* c, int tick, int t) {
+  if (t != 0) return;
+  if (tick == kTickBegin) clock_begin(c);
+  if (tick == kTickEnd) clock_end(c);
+}
+
 // One-pass halo fill of one grid (halo_shell_elem, swc_halo.cuh).
 template <typename T>
 __global__ void halo_periodic_kernel(const HaloArgs a, int total,
-                                     int clamp_x, int clamp_y, int clamp_z) {
+                                     int clamp_x, int clamp_y, int clamp_z,
+                                     SwcClock* clock, int tick) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  clock_tick(clock, tick, t);
   if (t < total) halo_shell_elem<T>(a, t, clamp_x, clamp_y, clamp_z);
 }
 
 // One-pass halo fill composing periodic, Dirichlet and Neumann sides
 // (halo_shell_bc_elem, swc_halo.cuh).
 template <typename T>
-__global__ void halo_shell_kernel(const ShellArgs a, int total) {
+__global__ void halo_shell_kernel(const ShellArgs a, int total,
+                                  SwcClock* clock, int tick) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  clock_tick(clock, tick, t);
   if (t < total) halo_shell_bc_elem<T>(a, t);
+}
+
+// Copy of every field with its halos filled (halo_copy_elem, swc_halo.cuh):
+// the fields of a functional call, which stay as they are. Memory bound. One
+// launch reads and writes each field once; a copy per field, the fill and a
+// memset per right-hand side were twelve launches, and their host time was
+// most of a small call (a right-hand side at 61 x 47 x 33: 101 us).
+template <typename T>
+__global__ void __launch_bounds__(kCopyY* kCopyX)
+    halo_copy_kernel(const ShellArgs a, const ShellCopy c) {
+  const int cy = blockIdx.x * kCopyY + threadIdx.x;
+  const int cx = blockIdx.y * kCopyX + threadIdx.y;
+  if (cy < a.ny + 2 * a.h && cx < a.nx + 2 * a.h)
+    halo_copy_elem<T>(a, c, cx, cy, blockIdx.z);
 }
 
 // ---------------------------------------------------------------------------
@@ -486,19 +515,20 @@ int swc_last_error(char* buf, size_t len) {
 
 int64_t swc_launch_count(void) { return g_launches; }
 
-int swc_halo_fill(const SwcGrid* grid, int32_t dtype, int32_t nfields,
-                  void* const* fields, const SwcFieldBC* bcs,
-                  int32_t rho_index, void* stream) {
-  swc::NvtxRange nvtx_range_("swc_halo_fill");
-  int st = check_grid(grid);
+// Checks of a halo fill's arguments; any_prim: a field whose conditions act on
+// its primitive.
+static int check_halo(const SwcGrid* grid, int32_t dtype, int32_t nfields,
+                      const void* const* fields, const SwcFieldBC* bcs,
+                      int32_t rho_index, bool* any_prim) {
+  const int st = check_grid(grid);
   if (st) return st;
   if (!dtype_ok(dtype)) return fail(SWC_ERR_ARG, "bad dtype %d", dtype);
   if (nfields <= 0 || nfields > SWC_MAX_FIELDS || !fields || !bcs)
     return fail(SWC_ERR_ARG, "bad field list (n=%d)", nfields);
-  bool any_prim = false;
+  *any_prim = false;
   for (int i = 0; i < nfields; ++i) {
     if (!fields[i]) return fail(SWC_ERR_ARG, "field %d is NULL", i);
-    if (bcs[i].via_primitive) any_prim = true;
+    if (bcs[i].via_primitive) *any_prim = true;
     for (int d = 0; d < 3; ++d)
       for (int s = 0; s < 2; ++s) {
         const SwcBC& b = bcs[i].side[d][s];
@@ -509,12 +539,55 @@ int swc_halo_fill(const SwcGrid* grid, int32_t dtype, int32_t nfields,
           return fail(SWC_ERR_ARG, "per-layer Dirichlet without planes");
       }
   }
-  if (any_prim && (rho_index < 0 || rho_index >= nfields))
+  if (*any_prim && (rho_index < 0 || rho_index >= nfields))
     return fail(SWC_ERR_ARG, "primitive BC needs rho (index %d)", rho_index);
+  return SWC_OK;
+}
+
+// The arguments of a one-pass fill (halo_shell_value), where one pass gives
+// what the three give: every side periodic, Dirichlet or Neumann, no
+// condition on a primitive variable, no periodic dim narrower than the halo.
+static bool shell_args(const SwcGrid* grid, int nfields,
+                       const void* const* fields, const SwcFieldBC* bcs,
+                       bool any_prim, ShellArgs& sa) {
+  const int h = grid->halo;
+  if (any_prim) return false;
+  memset(&sa, 0, sizeof(sa));
+  sa.nf = nfields;
+  const int nd[3] = {grid->nx, grid->ny, grid->nz};
+  for (int i = 0; i < nfields; ++i) {
+    sa.fld[i].f = const_cast<void*>(fields[i]);
+    for (int d = 0; d < 3; ++d) {
+      SwcBC lo = bcs[i].side[d][0], hi = bcs[i].side[d][1];
+      if (lo.kind == SWC_BC_PERIODIC || hi.kind == SWC_BC_PERIODIC) {
+        // A periodic side makes the whole dim periodic (boundary.py:65-68).
+        lo.kind = hi.kind = SWC_BC_PERIODIC;
+        if (nd[d] < h) return false;
+      } else if (lo.kind == SWC_BC_NONE || hi.kind == SWC_BC_NONE) {
+        return false;
+      }
+      sa.fld[i].bc[d][0] = lo;
+      sa.fld[i].bc[d][1] = hi;
+    }
+  }
+  sa.nx = grid->nx; sa.ny = grid->ny; sa.nz = grid->nz; sa.h = h;
+  sa.sx = grid->sx; sa.sz = grid->sz;
+  return true;
+}
+
+// swc_halo_fill, and the clock's tick in the fill's launch where that is one
+// pass, else in a launch of its own.
+static int halo_fill(const SwcGrid* grid, int32_t dtype, int32_t nfields,
+                     void* const* fields, const SwcFieldBC* bcs,
+                     int32_t rho_index, SwcClock* clock, int tick,
+                     void* stream) {
+  swc::NvtxRange nvtx_range_("swc_halo_fill");
+  bool any_prim = false;
+  int st = check_halo(grid, dtype, nfields, fields, bcs, rho_index, &any_prim);
+  if (st) return st;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int h = grid->halo;
-  if (h == 0) return SWC_OK;
-  {
+  if (h > 0) {
     // Every dim periodic for every field, or zero-gradient for every
     // field, no primitive BCs, halos no wider than the interior: one pass
     // instead of three.
@@ -549,49 +622,32 @@ int swc_halo_fill(const SwcGrid* grid, int32_t dtype, int32_t nfields,
       const unsigned blocks = (unsigned)((total + threads - 1) / threads);
       if (dtype == SWC_F32)
         halo_periodic_kernel<float><<<blocks, threads, 0, s>>>(
-            a, (int)total, clamp[0], clamp[1], clamp[2]);
+            a, (int)total, clamp[0], clamp[1], clamp[2], clock, tick);
       else
         halo_periodic_kernel<double><<<blocks, threads, 0, s>>>(
-            a, (int)total, clamp[0], clamp[1], clamp[2]);
+            a, (int)total, clamp[0], clamp[1], clamp[2], clock, tick);
       note_launch();
       return check_launch("halo_fill");
     }
-    // Every side periodic, Dirichlet or Neumann, none on a primitive
-    // variable, no periodic dim narrower than the halo: one pass that
-    // composes the three (bit for bit the same values).
-    bool one_pass = !any_prim && total < (1LL << 31);
+    // One pass that composes the three (bit for bit the same values).
     ShellArgs sa;
-    memset(&sa, 0, sizeof(sa));
-    sa.nf = nfields;
-    const int nd[3] = {grid->nx, grid->ny, grid->nz};
-    for (int i = 0; i < nfields && one_pass; ++i) {
-      sa.fld[i].f = fields[i];
-      for (int d = 0; d < 3 && one_pass; ++d) {
-        SwcBC lo = bcs[i].side[d][0], hi = bcs[i].side[d][1];
-        if (lo.kind == SWC_BC_PERIODIC || hi.kind == SWC_BC_PERIODIC) {
-          // A periodic side makes the whole dim periodic (boundary.py:65-68).
-          lo.kind = hi.kind = SWC_BC_PERIODIC;
-          if (nd[d] < h) one_pass = false;
-        } else if (lo.kind == SWC_BC_NONE || hi.kind == SWC_BC_NONE) {
-          one_pass = false;
-        }
-        sa.fld[i].bc[d][0] = lo;
-        sa.fld[i].bc[d][1] = hi;
-      }
-    }
-    if (one_pass) {
-      sa.nx = grid->nx; sa.ny = grid->ny; sa.nz = grid->nz; sa.h = h;
-      sa.sx = grid->sx; sa.sz = grid->sz;
+    if (total < (1LL << 31) &&
+        shell_args(grid, nfields, fields, bcs, any_prim, sa)) {
       const int threads = 256;
       const unsigned blocks = (unsigned)((total + threads - 1) / threads);
       if (dtype == SWC_F32)
-        halo_shell_kernel<float><<<blocks, threads, 0, s>>>(sa, (int)total);
+        halo_shell_kernel<float><<<blocks, threads, 0, s>>>(sa, (int)total,
+                                                            clock, tick);
       else
-        halo_shell_kernel<double><<<blocks, threads, 0, s>>>(sa, (int)total);
+        halo_shell_kernel<double><<<blocks, threads, 0, s>>>(sa, (int)total,
+                                                             clock, tick);
       note_launch();
       return check_launch("halo_fill");
     }
   }
+  if (tick == kTickBegin && (st = swc_clock_begin_step(clock, stream))) return st;
+  if (tick == kTickEnd && (st = swc_clock_end_step(clock, stream))) return st;
+  if (h == 0) return SWC_OK;
   // Phase 0: fields with direct BCs; phase 1: fields with primitive BCs,
   // after rho is complete in all three dims.
   for (int phase = 0; phase < (any_prim ? 2 : 1); ++phase) {
@@ -633,6 +689,64 @@ int swc_halo_fill(const SwcGrid* grid, int32_t dtype, int32_t nfields,
     }
   }
   return SWC_OK;
+}
+
+int swc_halo_fill(const SwcGrid* grid, int32_t dtype, int32_t nfields,
+                  void* const* fields, const SwcFieldBC* bcs,
+                  int32_t rho_index, void* stream) {
+  return halo_fill(grid, dtype, nfields, fields, bcs, rho_index, nullptr,
+                   kTickNone, stream);
+}
+
+int swc_halo_copy(const SwcGrid* grid, int32_t dtype, int32_t nfields,
+                  const void* const* src, void* const* dst,
+                  void* const* clear, const SwcFieldBC* bcs,
+                  int32_t rho_index, void* stream) {
+  swc::NvtxRange nvtx_range_("swc_halo_copy");
+  bool any_prim = false;
+  int st = check_halo(grid, dtype, nfields, src, bcs, rho_index, &any_prim);
+  if (st) return st;
+  if (!dst) return fail(SWC_ERR_ARG, "dst is NULL");
+  for (int i = 0; i < nfields; ++i) {
+    if (!dst[i] || (clear && !clear[i]))
+      return fail(SWC_ERR_ARG, "halo copy: field %d is NULL", i);
+    for (int k = 0; k < nfields; ++k)
+      if (dst[i] == src[k] || (clear && (clear[i] == src[k] || clear[i] == dst[k])))
+        return fail(SWC_ERR_ARG, "halo copy: outputs must not alias inputs");
+  }
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const int h = grid->halo;
+  const long long nxa = grid->nx + 2LL * h, nya = grid->ny + 2LL * h,
+                  nza = grid->nz + 2LL * h;
+  ShellArgs sa;
+  const long long by = (nxa + kCopyX - 1) / kCopyX;
+  if (by <= 65535 && nza <= 65535 &&
+      shell_args(grid, nfields, src, bcs, any_prim, sa)) {
+    ShellCopy c;
+    memset(&c, 0, sizeof(c));
+    for (int i = 0; i < nfields; ++i) {
+      c.dst[i] = dst[i];
+      c.clear[i] = clear ? clear[i] : nullptr;
+    }
+    const dim3 blocks((unsigned)((nya + kCopyY - 1) / kCopyY), (unsigned)by,
+                      (unsigned)nza);
+    const dim3 threads(kCopyY, kCopyX);
+    if (dtype == SWC_F32) halo_copy_kernel<float><<<blocks, threads, 0, s>>>(sa, c);
+    else halo_copy_kernel<double><<<blocks, threads, 0, s>>>(sa, c);
+    note_launch();
+    return check_launch("halo_copy");
+  }
+  // Conditions on primitives, unfilled sides, periodic dims narrower than the
+  // halo: copies, then the fill's passes.
+  const size_t bytes = (size_t)(grid->sz * nza) * (dtype == SWC_F32 ? 4 : 8);
+  for (int i = 0; i < nfields; ++i) {
+    cudaError_t e = cudaMemcpyAsync(dst[i], src[i], bytes,
+                                    cudaMemcpyDeviceToDevice, s);
+    if (e == cudaSuccess && clear) e = cudaMemsetAsync(clear[i], 0, bytes, s);
+    if (e != cudaSuccess)
+      return fail(SWC_ERR_LAUNCH, "halo copy: %s", cudaGetErrorString(e));
+  }
+  return swc_halo_fill(grid, dtype, nfields, dst, bcs, rho_index, stream);
 }
 
 // Checks and the kernel arguments shared by swc_rk_stage and
@@ -1072,6 +1186,17 @@ int swc_rk_combine(int64_t n, int32_t dtype, int32_t mode, double c0,
   return check_launch("rk_combine");
 }
 
+// The plain stage, or the extended one where `ext` is given.
+static int run_stage(const SwcGrid* grid, const SwcScheme* scheme,
+                     const SwcStageExt* ext, const void* const* uk,
+                     const void* const* u0, void* const* uout, int32_t mode,
+                     double c0, double c1, const double* dt, void* stream) {
+  return ext ? swc_rk_stage_ext(grid, scheme, ext, uk, u0, uout, mode, c0, c1,
+                                dt, nullptr, stream)
+             : swc_rk_stage(grid, scheme, uk, u0, uout, mode, c0, c1, dt,
+                            nullptr, stream);
+}
+
 int swc_rk_step(const SwcGrid* grid, const SwcScheme* scheme,
                 const SwcFieldBC* bcs, int32_t order, void* const* u,
                 void* const* work, SwcClock* clock_dev, void* stream) {
@@ -1095,19 +1220,22 @@ int swc_rk_step(const SwcGrid* grid, const SwcScheme* scheme,
   }
   const double* dt = &clock_dev->dt;
   double* dtmin = &clock_dev->dtmin;
-  if ((st = swc_clock_begin_step(clock_dev, stream))) return st;
-  if ((st = swc_halo_fill(grid, scheme->dtype, 5, u, bcs, 0, stream))) return st;
+  if ((st = halo_fill(grid, scheme->dtype, 5, u, bcs, 0, clock_dev, kTickBegin,
+                      stream)))
+    return st;
   if ((st = swc_rk_stage(grid, scheme, (const void* const*)u, nullptr, w1,
                          SWC_OUT_EULER, 0.0, 0.0, dt, nullptr, stream)))
     return st;
-  if ((st = swc_halo_fill(grid, scheme->dtype, 5, w1, bcs, 0, stream)))
+  if ((st = halo_fill(grid, scheme->dtype, 5, w1, bcs, 0, clock_dev,
+                      order == 3 ? kTickNone : kTickEnd, stream)))
     return st;
   if (order == 3) {
     if ((st = swc_rk_stage(grid, scheme, (const void* const*)w1,
                            (const void* const*)u, w2, SWC_OUT_CONVEX, 0.75,
                            0.25, dt, nullptr, stream)))
       return st;
-    if ((st = swc_halo_fill(grid, scheme->dtype, 5, w2, bcs, 0, stream)))
+    if ((st = halo_fill(grid, scheme->dtype, 5, w2, bcs, 0, clock_dev, kTickEnd,
+                        stream)))
       return st;
     if ((st = swc_rk_stage(grid, scheme, (const void* const*)w2,
                            (const void* const*)u, u, SWC_OUT_CONVEX,
@@ -1119,7 +1247,65 @@ int swc_rk_step(const SwcGrid* grid, const SwcScheme* scheme,
                            dt, dtmin, stream)))
       return st;
   }
-  return swc_clock_end_step(clock_dev, stream);
+  return SWC_OK;
+}
+
+int swc_rhs(const SwcGrid* grid, const SwcScheme* scheme,
+            const SwcFieldBC* bcs, const SwcStageExt* ext,
+            const void* const* u, void* const* out, void* const* work,
+            void* stream) {
+  swc::NvtxRange nvtx_range_("swc_rhs");
+  if (!scheme || !bcs || !u || !out || !work)
+    return fail(SWC_ERR_ARG, "NULL argument");
+  const int ns = scheme->nscalars;
+  if (ns < 0 || ns > 3)
+    return fail(SWC_ERR_UNSUPPORTED, "%d transported scalars (at most 3)", ns);
+  const int st = swc_halo_copy(grid, scheme->dtype, 5 + ns, u, work, out, bcs,
+                               0, stream);
+  if (st) return st;
+  return run_stage(grid, scheme, ext, (const void* const*)work, nullptr, out,
+                   SWC_OUT_RHS, 0.0, 0.0, nullptr, stream);
+}
+
+int swc_rk_step_out(const SwcGrid* grid, const SwcScheme* scheme,
+                    const SwcFieldBC* bcs, const SwcStageExt* ext,
+                    int32_t order, const void* const* u, void* const* out,
+                    void* const* work, const double* dt, void* stream) {
+  swc::NvtxRange nvtx_range_("swc_rk_step_out");
+  if (!scheme || !bcs || !u || !out || !work)
+    return fail(SWC_ERR_ARG, "NULL argument");
+  if (order != 2 && order != 3)
+    return fail(SWC_ERR_UNSUPPORTED, "Runge-Kutta order %d is not implemented",
+                order);
+  const int ns = scheme->nscalars, dtype = scheme->dtype;
+  if (ns < 0 || ns > 3)
+    return fail(SWC_ERR_UNSUPPORTED, "%d transported scalars (at most 3)", ns);
+  const int nf = 5 + ns;
+  // The filled input, and the stage state that is not `out`: RK3 passes
+  // through out, w, out; RK2 through w, out.
+  void* const* u0 = work;
+  void* const* w = work + nf;
+  void* const* first = order == 3 ? out : w;
+  int st = swc_halo_copy(grid, dtype, nf, u, u0, nullptr, bcs, 0, stream);
+  if (st) return st;
+  const void* const* cu0 = (const void* const*)u0;
+  if ((st = run_stage(grid, scheme, ext, cu0, nullptr, first, SWC_OUT_EULER,
+                      0.0, 0.0, dt, stream)))
+    return st;
+  if ((st = swc_halo_fill(grid, dtype, nf, first, bcs, 0, stream))) return st;
+  if (order == 3) {
+    if ((st = run_stage(grid, scheme, ext, (const void* const*)out, cu0, w,
+                        SWC_OUT_CONVEX, 0.75, 0.25, dt, stream)))
+      return st;
+    if ((st = swc_halo_fill(grid, dtype, nf, w, bcs, 0, stream))) return st;
+    st = run_stage(grid, scheme, ext, (const void* const*)w, cu0, out,
+                   SWC_OUT_CONVEX, 1.0 / 3.0, 2.0 / 3.0, dt, stream);
+  } else {
+    st = run_stage(grid, scheme, ext, (const void* const*)w, cu0, out,
+                   SWC_OUT_AVERAGE, 0.5, 0.0, dt, stream);
+  }
+  if (st) return st;
+  return swc_halo_fill(grid, dtype, nf, out, bcs, 0, stream);
 }
 
 }  // extern "C"

@@ -259,13 +259,67 @@ struct ShellArgs {
   long long sx, sz;
 };
 
+// Filled value of field F at the padded cell (x, y, z) = c (interior cells:
+// the field's own). Reads interior cells and planes only.
 template <typename T>
-__device__ __forceinline__ void halo_shell_bc_elem(const ShellArgs& a, int t) {
+__device__ __forceinline__ T halo_shell_value(const ShellArgs& a,
+                                              const ShellField& F, int cx,
+                                              int cy, int cz) {
   const int h = a.h;
   const int n[3] = {a.nx, a.ny, a.nz};
   const int ext[3] = {a.nx + 2 * h, a.ny + 2 * h, a.nz + 2 * h};
-  int c0[3];
-  shell_cell(h, a.nx, a.ny, a.nz, t, c0[0], c0[1], c0[2]);
+  int c[3] = {cx, cy, cz};
+  // Neumann steps met on the way back: layers and side per dim.
+  int nl[3] = {0, 0, 0}, ns[3] = {0, 0, 0};
+  bool dir = false;
+  T val = T(0);
+#pragma unroll
+  for (int d = 2; d >= 0; --d) {
+    const int side = c[d] < h ? 0 : (c[d] >= n[d] + h ? 1 : -1);
+    if (side < 0) continue;
+    const SwcBC& b = side == 0 ? F.bc[d][0] : F.bc[d][1];
+    if (b.kind == SWC_BC_PERIODIC) {
+      c[d] = side == 0 ? c[d] + n[d] : c[d] - n[d];
+    } else if (b.kind == SWC_BC_NEUMANN) {
+      // Layer l lies l + 1 cells from the edge cell.
+      ns[d] = side;
+      nl[d] = side == 0 ? h - c[d] : c[d] - (n[d] + h) + 1;
+      c[d] = side == 0 ? h : n[d] + h - 1;
+    } else {
+      // Dirichlet: layer 0 is the outermost on the low side, the
+      // innermost on the high side; planes are [halo][A][B] with (A, B)
+      // the other two dims in storage order (z, x, y).
+      const int l = side == 0 ? c[d] : c[d] - n[d] - h;
+      if (b.per_layer) {
+        int ia, ib, na, nb;
+        if (d == 0) { ia = c[2]; ib = c[1]; na = ext[2]; nb = ext[1]; }
+        else if (d == 1) { ia = c[2]; ib = c[0]; na = ext[2]; nb = ext[0]; }
+        else { ia = c[0]; ib = c[1]; na = ext[0]; nb = ext[1]; }
+        val = static_cast<const T*>(b.planes)[(long long)l * na * nb +
+                                              (long long)ia * nb + ib];
+      } else {
+        val = T(b.value);
+      }
+      dir = true;
+      break;
+    }
+  }
+  if (!dir)
+    val = static_cast<const T*>(F.f)[c[2] * a.sz + c[0] * a.sx + c[1]];
+  // Forwards: the Neumann steps in pass order x, y, z (only dims after a
+  // Dirichlet one were walked, so only those have steps).
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const T inc = T(ns[d] == 0 ? F.bc[d][0].value : F.bc[d][1].value);
+    for (int l = 0; l < nl[d]; ++l) val = ns[d] == 0 ? val - inc : val + inc;
+  }
+  return val;
+}
+
+template <typename T>
+__device__ __forceinline__ void halo_shell_bc_elem(const ShellArgs& a, int t) {
+  int cx, cy, cz;
+  shell_cell(a.h, a.nx, a.ny, a.nz, t, cx, cy, cz);
   // Every load before any store (the compiler cannot tell the fields
   // apart); the loads are of interior cells and planes, which no thread
   // writes.
@@ -273,58 +327,45 @@ __device__ __forceinline__ void halo_shell_bc_elem(const ShellArgs& a, int t) {
 #pragma unroll
   for (int fi = 0; fi < SWC_MAX_FIELDS; ++fi) {
     if (fi >= a.nf) break;
-    const ShellField& F = a.fld[fi];
-    int c[3] = {c0[0], c0[1], c0[2]};
-    // Neumann steps met on the way back: layers and side per dim.
-    int nl[3] = {0, 0, 0}, ns[3] = {0, 0, 0};
-    bool dir = false;
-    T val = T(0);
-#pragma unroll
-    for (int d = 2; d >= 0; --d) {
-      const int side = c[d] < h ? 0 : (c[d] >= n[d] + h ? 1 : -1);
-      if (side < 0) continue;
-      const SwcBC& b = side == 0 ? F.bc[d][0] : F.bc[d][1];
-      if (b.kind == SWC_BC_PERIODIC) {
-        c[d] = side == 0 ? c[d] + n[d] : c[d] - n[d];
-      } else if (b.kind == SWC_BC_NEUMANN) {
-        // Layer l lies l + 1 cells from the edge cell.
-        ns[d] = side;
-        nl[d] = side == 0 ? h - c[d] : c[d] - (n[d] + h) + 1;
-        c[d] = side == 0 ? h : n[d] + h - 1;
-      } else {
-        // Dirichlet: layer 0 is the outermost on the low side, the
-        // innermost on the high side; planes are [halo][A][B] with (A, B)
-        // the other two dims in storage order (z, x, y).
-        const int l = side == 0 ? c[d] : c[d] - n[d] - h;
-        if (b.per_layer) {
-          int ia, ib, na, nb;
-          if (d == 0) { ia = c[2]; ib = c[1]; na = ext[2]; nb = ext[1]; }
-          else if (d == 1) { ia = c[2]; ib = c[0]; na = ext[2]; nb = ext[0]; }
-          else { ia = c[0]; ib = c[1]; na = ext[0]; nb = ext[1]; }
-          val = static_cast<const T*>(b.planes)[(long long)l * na * nb +
-                                                (long long)ia * nb + ib];
-        } else {
-          val = T(b.value);
-        }
-        dir = true;
-        break;
-      }
-    }
-    if (!dir)
-      val = static_cast<const T*>(F.f)[c[2] * a.sz + c[0] * a.sx + c[1]];
-    // Forwards: the Neumann steps in pass order x, y, z (only dims after a
-    // Dirichlet one were walked, so only those have steps).
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      const T inc = T(ns[d] == 0 ? F.bc[d][0].value : F.bc[d][1].value);
-      for (int l = 0; l < nl[d]; ++l) val = ns[d] == 0 ? val - inc : val + inc;
-    }
-    v[fi] = val;
+    v[fi] = halo_shell_value<T>(a, a.fld[fi], cx, cy, cz);
   }
-  const long long o = c0[2] * a.sz + c0[0] * a.sx + c0[1];
+  const long long o = cz * a.sz + cx * a.sx + cy;
 #pragma unroll
   for (int fi = 0; fi < SWC_MAX_FIELDS; ++fi)
     if (fi < a.nf) static_cast<T*>(a.fld[fi].f)[o] = v[fi];
+}
+
+// Copies with filled halos: dst[f] of every padded cell takes what
+// halo_shell_bc_elem would leave in a copy of the field, which stays as it
+// is; `clear` (where not NULL) gets zeros in its halo cells, as a
+// right-hand side returns them.
+struct ShellCopy {
+  void* dst[SWC_MAX_FIELDS];
+  void* clear[SWC_MAX_FIELDS];
+};
+// A cell of the padded grid: 32 cells of a row along y by 8 rows per block.
+constexpr int kCopyY = 32, kCopyX = 8;
+
+template <typename T>
+__device__ __forceinline__ void halo_copy_elem(const ShellArgs& a,
+                                               const ShellCopy& c, int cx,
+                                               int cy, int cz) {
+  const int h = a.h;
+  const long long o = cz * a.sz + cx * a.sx + cy;
+  const bool halo = cx < h || cx >= a.nx + h || cy < h || cy >= a.ny + h ||
+                    cz < h || cz >= a.nz + h;
+  T v[SWC_MAX_FIELDS];
+#pragma unroll
+  for (int f = 0; f < SWC_MAX_FIELDS; ++f)
+    if (f < a.nf)
+      v[f] = halo ? halo_shell_value<T>(a, a.fld[f], cx, cy, cz)
+                  : static_cast<const T*>(a.fld[f].f)[o];
+#pragma unroll
+  for (int f = 0; f < SWC_MAX_FIELDS; ++f)
+    if (f < a.nf) {
+      static_cast<T*>(c.dst[f])[o] = v[f];
+      if (halo && c.clear[f]) static_cast<T*>(c.clear[f])[o] = T(0);
+    }
 }
 
 // Cells of the halo shell of an (nx, ny, nz) grid with halo h.

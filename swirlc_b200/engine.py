@@ -386,12 +386,8 @@ class Solver:
             dt: Optional[torch.Tensor] = None,
             dtmin_out: Optional[torch.Tensor] = None,
             helper: Optional[Dict[str, torch.Tensor]] = None) -> None:
-    if self.use_ext or helper:
-      e = self.ext
-      if helper:
-        e = nat.SwcStageExt.from_buffer_copy(self.ext)
-        e.p_ref = self._helper_field(helper, 'p_ref').data_ptr()
-        e.rho_ref = self._helper_field(helper, 'rho_ref').data_ptr()
+    e = self._ext_of(helper)
+    if e is not None:
       nat.check(nat.load().swc_rk_stage_ext(
           ctypes.byref(self.grid), ctypes.byref(self.scheme), ctypes.byref(e),
           nat.ptr_array(uk), nat.ptr_array(u0) if u0 is not None else None,
@@ -478,18 +474,65 @@ class Solver:
     return [alloc(self.shape, dtype=self.dtype, device=self.device)
             for _ in range(len(self.names))]
 
+  # ---------------------------------------------------- functional forms
+  # One library call each (swc_rhs, swc_rk_step_out): the copy that leaves the
+  # caller's fields alone fills the halos too, and the work states are one
+  # allocation. With replicas the halos come from other ranks between the
+  # stages, so the steps are composed here.
+  def _ext_of(self, helper):
+    """The stage's SwcStageExt, or None for the plain stage."""
+    if helper:
+      e = nat.SwcStageExt.from_buffer_copy(self.ext)
+      e.p_ref = self._helper_field(helper, 'p_ref').data_ptr()
+      e.rho_ref = self._helper_field(helper, 'rho_ref').data_ptr()
+      return e
+    return self.ext if self.use_ext else None
+
+  def _work(self, states: int):
+    """(tensor that holds it, addresses) of uninitialised scratch for `states`
+    states; fields start 256 bytes apart at the least multiple."""
+    nf = len(self.names)
+    esz = 4 if self.dtype == torch.float32 else 8
+    field = (self.shape[0] * self.shape[1] * self.shape[2] * esz + 255) // 256 * 256
+    block = torch.empty(states * nf * field, dtype=torch.uint8,
+                        device=self.device)
+    base = block.data_ptr()
+    return block, nat.addr_array([base + i * field for i in range(states * nf)])
+
   def rhs(self, fields: Sequence[torch.Tensor],
           helper: Optional[Dict[str, torch.Tensor]] = None) -> List[torch.Tensor]:
     """Functional RHS: copies, fills halos of the copy, returns dU/dt."""
-    work = [f.clone() for f in fields]
-    self.fill_halos(work)
-    out = self.new_fields(zero=True)
-    self.stage(work, None, out, nat.SWC_OUT_RHS, helper=helper)
+    if self._layout is not None:
+      work = [f.clone() for f in fields]
+      self.fill_halos(work)
+      out = self.new_fields(zero=True)
+      self.stage(work, None, out, nat.SWC_OUT_RHS, helper=helper)
+      return out
+    u = [f.contiguous() for f in fields]
+    ext = self._ext_of(helper)
+    out = self.new_fields(zero=False)
+    block, work = self._work(1)
+    nat.check(nat.load().swc_rhs(
+        self.grid, self.scheme, self.bcs, ext, nat.ptr_array(u),
+        nat.ptr_array(out), work, nat.stream_ptr()), 'rhs')
+    return out
+
+  def _step_out(self, order: int, fields, dt: float, helper):
+    u = [f.contiguous() for f in fields]
+    dtt = self.dt_tensor(dt)
+    ext = self._ext_of(helper)
+    out = self.new_fields(zero=False)
+    block, work = self._work(2)
+    nat.check(nat.load().swc_rk_step_out(
+        self.grid, self.scheme, self.bcs, ext, order, nat.ptr_array(u),
+        nat.ptr_array(out), work, dtt.data_ptr(), nat.stream_ptr()), 'rk step')
     return out
 
   def rk3(self, fields: Sequence[torch.Tensor], dt: float,
           helper: Optional[Dict[str, torch.Tensor]] = None) -> List[torch.Tensor]:
     """Functional SSP-RK3 step (rk3.py:87-120) returning new fields."""
+    if self._layout is None:
+      return self._step_out(3, fields, dt, helper)
     dtt = self.dt_tensor(dt)
     u0 = [f.clone() for f in fields]
     self.fill_halos(u0)
@@ -508,6 +551,8 @@ class Solver:
   def rk2(self, fields: Sequence[torch.Tensor], dt: float,
           helper: Optional[Dict[str, torch.Tensor]] = None) -> List[torch.Tensor]:
     """Functional RK2 step (rk2.py:63-86) returning new fields."""
+    if self._layout is None:
+      return self._step_out(2, fields, dt, helper)
     dtt = self.dt_tensor(dt)
     u0 = [f.clone() for f in fields]
     self.fill_halos(u0)
