@@ -113,13 +113,27 @@ __global__ void halo_shell_kernel(const ShellArgs a, int total,
 // launch reads and writes each field once; a copy per field, the fill and a
 // memset per right-hand side were twelve launches, and their host time was
 // most of a small call (a right-hand side at 61 x 47 x 33: 101 us).
-template <typename T>
+template <typename T, int NF>
 __global__ void __launch_bounds__(kCopyY* kCopyX)
     halo_copy_kernel(const ShellArgs a, const ShellCopy c) {
   const int cy = blockIdx.x * kCopyY + threadIdx.x;
-  const int cx = blockIdx.y * kCopyX + threadIdx.y;
-  if (cy < a.ny + 2 * a.h && cx < a.nx + 2 * a.h)
-    halo_copy_elem<T>(a, c, cx, cy, blockIdx.z);
+  const int cx = blockIdx.y * kCopyX * kCopyRows + threadIdx.y;
+  if (cy < a.ny + 2 * a.h) halo_copy_elem<T, NF>(a, c, cx, cy, blockIdx.z);
+}
+template <typename T>
+void launch_halo_copy(const ShellArgs& a, const ShellCopy& c, dim3 blocks,
+                      cudaStream_t s) {
+  const dim3 t(kCopyY, kCopyX);
+  switch (a.nf) {
+    case 1: halo_copy_kernel<T, 1><<<blocks, t, 0, s>>>(a, c); break;
+    case 2: halo_copy_kernel<T, 2><<<blocks, t, 0, s>>>(a, c); break;
+    case 3: halo_copy_kernel<T, 3><<<blocks, t, 0, s>>>(a, c); break;
+    case 4: halo_copy_kernel<T, 4><<<blocks, t, 0, s>>>(a, c); break;
+    case 5: halo_copy_kernel<T, 5><<<blocks, t, 0, s>>>(a, c); break;
+    case 6: halo_copy_kernel<T, 6><<<blocks, t, 0, s>>>(a, c); break;
+    case 7: halo_copy_kernel<T, 7><<<blocks, t, 0, s>>>(a, c); break;
+    default: halo_copy_kernel<T, 8><<<blocks, t, 0, s>>>(a, c); break;
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -570,6 +584,18 @@ static bool shell_args(const SwcGrid* grid, int nfields,
       sa.fld[i].bc[d][1] = hi;
     }
   }
+  for (int d = 0; d < 3; ++d) {
+    int wrap = 0, clamp = 0;
+    for (int i = 0; i < nfields; ++i) {
+      const SwcBC* b = sa.fld[i].bc[d];
+      if (b[0].kind == SWC_BC_PERIODIC) ++wrap;
+      if (b[0].kind == SWC_BC_NEUMANN && b[1].kind == SWC_BC_NEUMANN &&
+          b[0].value == 0.0 && b[1].value == 0.0)
+        ++clamp;
+    }
+    sa.dims[d] = wrap == nfields ? kShellWrap
+                                 : clamp == nfields ? kShellClamp : kShellMixed;
+  }
   sa.nx = grid->nx; sa.ny = grid->ny; sa.nz = grid->nz; sa.h = h;
   sa.sx = grid->sx; sa.sz = grid->sz;
   return true;
@@ -719,7 +745,8 @@ int swc_halo_copy(const SwcGrid* grid, int32_t dtype, int32_t nfields,
   const long long nxa = grid->nx + 2LL * h, nya = grid->ny + 2LL * h,
                   nza = grid->nz + 2LL * h;
   ShellArgs sa;
-  const long long by = (nxa + kCopyX - 1) / kCopyX;
+  const int rows = kCopyX * kCopyRows;
+  const long long by = (nxa + rows - 1) / rows;
   if (by <= 65535 && nza <= 65535 &&
       shell_args(grid, nfields, src, bcs, any_prim, sa)) {
     ShellCopy c;
@@ -730,9 +757,8 @@ int swc_halo_copy(const SwcGrid* grid, int32_t dtype, int32_t nfields,
     }
     const dim3 blocks((unsigned)((nya + kCopyY - 1) / kCopyY), (unsigned)by,
                       (unsigned)nza);
-    const dim3 threads(kCopyY, kCopyX);
-    if (dtype == SWC_F32) halo_copy_kernel<float><<<blocks, threads, 0, s>>>(sa, c);
-    else halo_copy_kernel<double><<<blocks, threads, 0, s>>>(sa, c);
+    if (dtype == SWC_F32) launch_halo_copy<float>(sa, c, blocks, s);
+    else launch_halo_copy<double>(sa, c, blocks, s);
     note_launch();
     return check_launch("halo_copy");
   }

@@ -257,7 +257,30 @@ struct ShellArgs {
   ShellField fld[SWC_MAX_FIELDS];
   int nx, ny, nz, h;
   long long sx, sz;
+  // Per dim: kShellWrap where every field is periodic, kShellClamp where every
+  // field has Neumann sides of slope 0, else kShellMixed.
+  int dims[3];
 };
+enum { kShellMixed, kShellWrap, kShellClamp };
+
+// Offset of the interior cell that every field copies at the padded cell
+// (cx, cy, cz) (its own for an interior cell). False where the cell lies in
+// the halo of a mixed dim: there the fields take halo_shell_value, whose walk
+// per field costs some ten times as much.
+__device__ __forceinline__ bool shell_source(const ShellArgs& a, int cx, int cy,
+                                             int cz, long long& os) {
+  const int h = a.h;
+  bool same = true;
+  auto src = [&](int c, int n, int kind) {
+    if (c >= h && c < n + h) return c;
+    if (kind == kShellMixed) same = false;
+    if (kind == kShellWrap) return c < h ? c + n : c - n;
+    return c < h ? h : n + h - 1;
+  };
+  const int x = src(cx, a.nx, a.dims[0]), y = src(cy, a.ny, a.dims[1]);
+  os = src(cz, a.nz, a.dims[2]) * a.sz + x * a.sx + y;
+  return same;
+}
 
 // Filled value of field F at the padded cell (x, y, z) = c (interior cells:
 // the field's own). Reads interior cells and planes only.
@@ -324,10 +347,15 @@ __device__ __forceinline__ void halo_shell_bc_elem(const ShellArgs& a, int t) {
   // apart); the loads are of interior cells and planes, which no thread
   // writes.
   T v[SWC_MAX_FIELDS];
+  long long os;
+  if (shell_source(a, cx, cy, cz, os)) {
 #pragma unroll
-  for (int fi = 0; fi < SWC_MAX_FIELDS; ++fi) {
-    if (fi >= a.nf) break;
-    v[fi] = halo_shell_value<T>(a, a.fld[fi], cx, cy, cz);
+    for (int fi = 0; fi < SWC_MAX_FIELDS; ++fi)
+      if (fi < a.nf) v[fi] = static_cast<const T*>(a.fld[fi].f)[os];
+  } else {
+#pragma unroll
+    for (int fi = 0; fi < SWC_MAX_FIELDS; ++fi)
+      if (fi < a.nf) v[fi] = halo_shell_value<T>(a, a.fld[fi], cx, cy, cz);
   }
   const long long o = cz * a.sz + cx * a.sx + cy;
 #pragma unroll
@@ -337,35 +365,52 @@ __device__ __forceinline__ void halo_shell_bc_elem(const ShellArgs& a, int t) {
 
 // Copies with filled halos: dst[f] of every padded cell takes what
 // halo_shell_bc_elem would leave in a copy of the field, which stays as it
-// is; `clear` (where not NULL) gets zeros in its halo cells, as a
-// right-hand side returns them.
+// is; `clear` (where not NULL, for all fields or none) gets zeros in its halo
+// cells, as a right-hand side returns them.
 struct ShellCopy {
   void* dst[SWC_MAX_FIELDS];
   void* clear[SWC_MAX_FIELDS];
 };
-// A cell of the padded grid: 32 cells of a row along y by 8 rows per block.
-constexpr int kCopyY = 32, kCopyX = 8;
+// A block of 32 x 8 threads takes 32 cells along y by 16 rows, two per thread.
+constexpr int kCopyY = 32, kCopyX = 8, kCopyRows = 2;
 
-template <typename T>
+// The cells (cx + k * kCopyX, cy, cz), k < kCopyRows, of the padded grid. The
+// loads of all cells with one source for every field come before any store,
+// so that they are in flight together.
+template <typename T, int NF>
 __device__ __forceinline__ void halo_copy_elem(const ShellArgs& a,
                                                const ShellCopy& c, int cx,
                                                int cy, int cz) {
-  const int h = a.h;
-  const long long o = cz * a.sz + cx * a.sx + cy;
-  const bool halo = cx < h || cx >= a.nx + h || cy < h || cy >= a.ny + h ||
-                    cz < h || cz >= a.nz + h;
-  T v[SWC_MAX_FIELDS];
+  const int h = a.h, nxa = a.nx + 2 * h;
+  const bool yz = cy < h || cy >= a.ny + h || cz < h || cz >= a.nz + h;
+  T v[kCopyRows][NF];
+  bool same[kCopyRows];
 #pragma unroll
-  for (int f = 0; f < SWC_MAX_FIELDS; ++f)
-    if (f < a.nf)
-      v[f] = halo ? halo_shell_value<T>(a, a.fld[f], cx, cy, cz)
-                  : static_cast<const T*>(a.fld[f].f)[o];
+  for (int k = 0; k < kCopyRows; ++k) {
+    const int x = cx + k * kCopyX;
+    long long os;
+    same[k] = x < nxa && shell_source(a, x, cy, cz, os);
 #pragma unroll
-  for (int f = 0; f < SWC_MAX_FIELDS; ++f)
-    if (f < a.nf) {
-      static_cast<T*>(c.dst[f])[o] = v[f];
-      if (halo && c.clear[f]) static_cast<T*>(c.clear[f])[o] = T(0);
+    for (int f = 0; f < NF; ++f)
+      if (same[k]) v[k][f] = static_cast<const T*>(a.fld[f].f)[os];
+  }
+#pragma unroll
+  for (int k = 0; k < kCopyRows; ++k) {
+    const int x = cx + k * kCopyX;
+    if (x >= nxa) continue;
+    if (!same[k]) {
+#pragma unroll
+      for (int f = 0; f < NF; ++f)
+        v[k][f] = halo_shell_value<T>(a, a.fld[f], x, cy, cz);
     }
+    const long long o = cz * a.sz + x * a.sx + cy;
+    if (c.clear[0] && (yz || x < h || x >= a.nx + h)) {
+#pragma unroll
+      for (int f = 0; f < NF; ++f) static_cast<T*>(c.clear[f])[o] = T(0);
+    }
+#pragma unroll
+    for (int f = 0; f < NF; ++f) static_cast<T*>(c.dst[f])[o] = v[k][f];
+  }
 }
 
 // Cells of the halo shell of an (nx, ny, nz) grid with halo h.
