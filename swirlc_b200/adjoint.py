@@ -102,10 +102,8 @@ class RunAdjoint:
         self._tmp = self._new_buffers()
       buf = self._tmp
     dtt = self._dt_dev[i:i + 1]
-    s.fill_halos(u)
     u0, w1 = buf[0], buf[1]
-    for a, b in zip(u0, u):
-      a.copy_(b)
+    s.copy_filled(u, u0)
     s.stage(u0, None, w1, nat.SWC_OUT_EULER, dt=dtt)
     s.fill_halos(w1)
     if self.order == 3:

@@ -35,9 +35,15 @@ namespace {
 // Reverse of recon_cell<0, O> (swc_physics.cuh) on one or two variables
 // (the lanes of O): both WENO5 face values of the cell v[2] from
 // v[0..4] = v[c-2 .. c+2], which share the smoothness indicators.
-// vb[k] += d right/dv[k] * rb + d left/dv[k] * lb. Per stencil r:
-// a_r = sum A[r][k] v[k], b_r = sum Bc[r][k] v[k],
-// beta_r = 13/12 a_r^2 + 1/4 b_r^2 + eps, candidate q_r = sum Q[r][k] v[k].
+// vb[k] += d right/dv[k] * rb + d left/dv[k] * lb. The forward is that of
+// weno5_right_v / weno5_left_v: first differences e, second differences f,
+// third differences t_lo, t_up, B_r = 13/3 a_r^2 + b_r^2 + 4 eps,
+// w_r = 1/B_r^2 and each face value a central candidate plus num / den. With
+// c = num / den and g = cotangent / den of a face (den with the sign of the
+// correction, as there), d num = g and d den = -g c; the differences'
+// cotangents move onto the cells last. 92 products and sums and 5
+// reciprocals per cell, against 150 with the three candidates of each face
+// spelled out.
 template <class O>
 __device__ __forceinline__ void weno5_cell_vjp_v(const typename O::V* v,
                                                  typename O::V rb,
@@ -45,85 +51,55 @@ __device__ __forceinline__ void weno5_cell_vjp_v(const typename O::V* v,
                                                  typename O::V* vb) {
   using S = typename O::S;
   using V = typename O::V;
-  constexpr double A[3][5] = {{0, 0, 1, -2, 1}, {0, 1, -2, 1, 0}, {1, -2, 1, 0, 0}};
-  constexpr double Bc[3][5] = {{0, 0, 3, -4, 1}, {0, 1, 0, -1, 0}, {1, -4, 3, 0, 0}};
-  constexpr double QR[3][5] = {{0, 0, 1.0 / 3, 5.0 / 6, -1.0 / 6},
-                               {0, -1.0 / 6, 5.0 / 6, 1.0 / 3, 0},
-                               {1.0 / 3, -7.0 / 6, 11.0 / 6, 0, 0}};
-  constexpr double QL[3][5] = {{0, 0, 11.0 / 6, -7.0 / 6, 1.0 / 3},
-                               {0, 1.0 / 3, 5.0 / 6, -1.0 / 6, 0},
-                               {-1.0 / 6, 5.0 / 6, 1.0 / 3, 0, 0}};
-  constexpr double DR[3] = {0.3, 0.6, 0.1}, DL[3] = {0.1, 0.6, 0.3};
-  // acc + c x with c a nonzero stencil coefficient (c = +-1 as an add).
-  auto term = [](double c, V x, V acc, bool first) -> V {
-    if (first) return c == 1 ? x : O::mul(O::splat(S(c)), x);
-    if (c == 1) return O::add(acc, x);
-    if (c == -1) return O::sub(acc, x);
-    return O::fma(O::splat(S(c)), x, acc);
-  };
-  auto lin = [&](const double* c) -> V {
-    V acc = O::splat(S(0));
-    bool first = true;
-#pragma unroll
-    for (int k = 0; k < 5; ++k)
-      if (c[k] != 0) {
-        acc = term(c[k], v[k], acc, first);
-        first = false;
-      }
-    return acc;
-  };
-  const V c1312 = O::splat(S(13.0 / 12.0)), eps = O::splat(S(1e-6));
-  V av[3], bv[3], ib[3], iq[3], qr[3], ql[3];
-  V sr, sl, nr, nl;
-#pragma unroll
-  for (int r = 0; r < 3; ++r) {
-    av[r] = lin(A[r]);
-    bv[r] = lin(Bc[r]);
-    qr[r] = lin(QR[r]);
-    ql[r] = lin(QL[r]);
-    const V be = O::add(O::fma(O::mul(c1312, av[r]), av[r],
-                               O::mul(O::mul(O::splat(S(0.25)), bv[r]), bv[r])),
-                        eps);
-    ib[r] = O::rcp(be);         // 1 / beta_r
-    iq[r] = O::mul(ib[r], ib[r]);  // 1 / beta_r^2
-    const V ar = O::mul(O::splat(S(DR[r])), iq[r]);
-    const V al = O::mul(O::splat(S(DL[r])), iq[r]);
-    if (r == 0) {
-      sr = ar;
-      sl = al;
-      nr = O::mul(ar, qr[r]);
-      nl = O::mul(al, ql[r]);
-    } else {
-      sr = O::add(sr, ar);
-      sl = O::add(sl, al);
-      nr = O::fma(ar, qr[r], nr);
-      nl = O::fma(al, ql[r], nl);
-    }
-  }
-  const V isr = O::rcp(sr), isl = O::rcp(sl);
-  const V outr = O::mul(nr, isr), outl = O::mul(nl, isl);
-  const V gr = O::mul(rb, isr), gl = O::mul(lb, isl);
-#pragma unroll
-  for (int r = 0; r < 3; ++r) {
-    // alpha_r = D_r / beta_r^2; out = sum alpha q / sum alpha.
-    const V gdr = O::mul(gr, O::splat(S(DR[r])));
-    const V gdl = O::mul(gl, O::splat(S(DL[r])));
-    const V qbr = O::mul(gdr, iq[r]);
-    const V qbl = O::mul(gdl, iq[r]);
-    const V ibq = O::fma(gdr, O::sub(qr[r], outr),
-                         O::mul(gdl, O::sub(ql[r], outl)));
-    // d(1/beta^2)/d beta = -2 / beta^3
-    const V bb = O::mul(O::mul(O::mul(O::splat(S(-2)), ibq), iq[r]), ib[r]);
-    const V ca = O::mul(O::mul(bb, O::splat(S(2.0 * 13.0 / 12.0))), av[r]);
-    const V cb = O::mul(O::mul(bb, O::splat(S(0.5))), bv[r]);
-#pragma unroll
-    for (int k = 0; k < 5; ++k) {
-      if (QR[r][k] != 0) vb[k] = O::fma(O::splat(S(QR[r][k])), qbr, vb[k]);
-      if (QL[r][k] != 0) vb[k] = O::fma(O::splat(S(QL[r][k])), qbl, vb[k]);
-      if (A[r][k] != 0) vb[k] = term(A[r][k], ca, vb[k], false);
-      if (Bc[r][k] != 0) vb[k] = term(Bc[r][k], cb, vb[k], false);
-    }
-  }
+  auto k = [](double c) -> V { return O::splat(S(c)); };
+  const V e0 = O::sub(v[1], v[0]), e1 = O::sub(v[2], v[1]);
+  const V e2 = O::sub(v[3], v[2]), e3 = O::sub(v[4], v[3]);
+  // a_2, a_1, a_0 of the candidates r = 2, 1, 0.
+  const V f0 = O::sub(e1, e0), f1 = O::sub(e2, e1), f2 = O::sub(e3, e2);
+  const V t_lo = O::sub(f1, f0), t_up = O::sub(f2, f1);
+  const V c0 = O::mul(k(13.0 / 3.0), f0), c1 = O::mul(k(13.0 / 3.0), f1);
+  const V c2 = O::mul(k(13.0 / 3.0), f2);
+  const V b0 = O::fma(k(-3), e2, e3), b1 = O::add(e2, e1);
+  const V b2 = O::fma(k(-3), e1, e0);
+  const V eps = k(4e-6);
+  const V i0 = O::rcp(O::fma(c2, f2, O::fma(b0, b0, eps)));
+  const V i1 = O::rcp(O::fma(c1, f1, O::fma(b1, b1, eps)));
+  const V i2 = O::rcp(O::fma(c0, f0, O::fma(b2, b2, eps)));
+  const V w0 = O::mul(i0, i0), w1 = O::mul(i1, i1), w2 = O::mul(i2, i2);
+  const V p0 = O::mul(w0, t_up), p2 = O::mul(w2, t_lo), m1 = O::mul(k(12), w1);
+  const V dr = O::rcp(O::fma(k(-6), w0, O::fma(k(-2), w2, O::mul(k(-1), m1))));
+  const V dl = O::rcp(O::fma(k(2), w0, O::fma(k(6), w2, m1)));
+  const V cr = O::mul(O::fma(k(2.0 / 3.0), p2, p0), dr);
+  const V cl = O::mul(O::fma(k(2.0 / 3.0), p0, p2), dl);
+  const V gr = O::mul(rb, dr), gl = O::mul(lb, dl);
+  const V hr = O::mul(gr, cr), hl = O::mul(gl, cl);
+  const V s0 = O::fma(k(2.0 / 3.0), gl, gr), s2 = O::fma(k(2.0 / 3.0), gr, gl);
+  // Cotangents of the weights, then x_r = 2 dB_r = -4 w_r / B_r dw_r.
+  const V y0 = O::fma(t_up, s0, O::fma(k(6), hr, O::mul(k(-2), hl)));
+  const V y1 = O::mul(k(12), O::sub(hr, hl));
+  const V y2 = O::fma(t_lo, s2, O::fma(k(2), hr, O::mul(k(-6), hl)));
+  const V x0 = O::mul(O::mul(k(-4), O::mul(w0, i0)), y0);
+  const V x1 = O::mul(O::mul(k(-4), O::mul(w1, i1)), y1);
+  const V x2 = O::mul(O::mul(k(-4), O::mul(w2, i2)), y2);
+  // Cotangents of t_up, t_lo, of the second and of the first differences.
+  const V tu = O::mul(w0, s0), tl = O::mul(w2, s2);
+  const V g0 = O::sub(O::mul(c0, x2), tl);
+  const V g1 = O::fma(c1, x1, O::sub(tl, tu));
+  const V g2 = O::fma(c2, x0, tu);
+  const V z0 = O::mul(b0, x0), z1 = O::mul(b1, x1), z2 = O::mul(b2, x2);
+  const V d0 = O::sub(z2, g0);
+  const V d1 = O::add(O::fma(k(-3), z2, z1),
+                      O::add(O::sub(g0, g1), O::fma(k(1.0 / 6.0), rb,
+                                                    O::mul(k(-1.0 / 3.0), lb))));
+  const V d2 = O::add(O::fma(k(-3), z0, z1),
+                      O::add(O::sub(g1, g2), O::fma(k(1.0 / 3.0), rb,
+                                                    O::mul(k(-1.0 / 6.0), lb))));
+  const V d3 = O::add(z0, g2);
+  vb[0] = O::sub(vb[0], d0);
+  vb[1] = O::add(vb[1], O::sub(d0, d1));
+  vb[2] = O::add(vb[2], O::add(O::add(rb, lb), O::sub(d1, d2)));
+  vb[3] = O::add(vb[3], O::sub(d2, d3));
+  vb[4] = O::add(vb[4], d3);
 }
 
 // Primitive cotangents of one face state, rotated frame (u[0] normal).
@@ -629,7 +605,7 @@ struct VjpArgs {
   int gravity_mask;
   double g[3];
   double* nu_bar;
-  int seg;  // faces per thread along a line
+  int seg[3];  // faces per thread along a line of face pass D
   int limiter;  // MUSCL limiter (SWC_LIM_*)
   // vout = alpha*lam + c1*x1 + c2*x2 + beta*H^T J^T lam on the interior.
   double alpha, c1, c2;
@@ -637,10 +613,11 @@ struct VjpArgs {
   const void* x2[5];
   // Per face pass D (in that pass's layout), so that every sum has a fixed
   // order: primitive cotangents of the five cells at the head of each
-  // segment (hb), the cotangents of each cell's four tangential differences
-  // (tg; tgh: the head cell's part from its segment's first face), and the
-  // nu cotangent of every block (nu_part, pass D from nu_off[D]).
-  // vjp_fix_kernel adds the first two to the primitive cotangents.
+  // segment but a line's first (hb), the cotangents of each cell's four
+  // tangential differences (tg; tgh: the head cell's part from its segment's
+  // first face), and the nu cotangent of every block (nu_part, pass D from
+  // nu_off[D]). vjp_cell_kernel adds the first two to the primitive
+  // cotangents.
   void* hb[3][7];
   void* tg[3][4];
   void* tgh[3][4];
@@ -661,13 +638,14 @@ __device__ __forceinline__ T pe_of(const VjpArgs& a, int xa, int ya, int za) {
 // cells of one z plane, 4 per thread; the transposed copies go through a
 // shared-memory tile so that both layouts are read and written coalesced.
 constexpr int TT = 32;
-// Faces per thread of a face pass. The five head cells of consecutive
-// segments must not overlap (vjp_fix_kernel adds each once).
-constexpr int kVjpSeg = 16;
-static_assert(kVjpSeg >= 5, "segment heads would overlap");
+// Fewest faces per thread of a face pass: the five head cells of consecutive
+// segments must not overlap (vjp_cell_kernel adds each once).
+constexpr int kVjpMinSeg = 5;
+// Threads per block of a face pass.
+constexpr int kVjpFaceThreads = 128;
 
-// Primitives of every cell (halos included), in both layouts, with their
-// cotangent buffers cleared, and lam transposed.
+// Primitives of every cell (halos included), in both layouts, and lam
+// transposed.
 // Dynamic shared memory of the transposing kernels: one [TT][TT+1] tile
 // per transposed variable, so a single barrier separates all writers from
 // all readers.
@@ -713,10 +691,7 @@ __global__ void __launch_bounds__(256) vjp_prim_kernel(const VjpArgs a) {
     if (xa >= nxa || ya >= nya) continue;
     const long long o = za * a.sz + xa * a.sx + ya;
 #pragma unroll
-    for (int v = 0; v < 7; ++v) {
-      static_cast<T*>(a.prim[v])[o] = pr[k][v];
-      static_cast<T*>(a.pbar[v])[o] = T(0);
-    }
+    for (int v = 0; v < 7; ++v) static_cast<T*>(a.prim[v])[o] = pr[k][v];
   }
   // tiles[v][x - x0][y - y0]; the transposed write reads them along x.
 #pragma unroll
@@ -735,20 +710,18 @@ __global__ void __launch_bounds__(256) vjp_prim_kernel(const VjpArgs a) {
       const int xa = x0 + tx, ya = y0 + yl;
       if (xa >= nxa || ya >= nya) continue;
       const long long ot = za * a.tsz + ya * a.tsy + xa;
-      if (v < 7) {
-        static_cast<T*>(a.primT[v])[ot] = tile[tx][yl];
-        static_cast<T*>(a.pbarT[v])[ot] = T(0);
-      } else {
-        static_cast<T*>(a.lamT[v - 7])[ot] = tile[tx][yl];
-      }
+      if (v < 7) static_cast<T*>(a.primT[v])[ot] = tile[tx][yl];
+      else static_cast<T*>(a.lamT[v - 7])[ot] = tile[tx][yl];
     }
   }
 }
 
 // Face VJPs along dim D. Thread = `seg` consecutive faces of one line along
 // D; a register window holds the 6-cell stencil primitives and their
-// cotangents, and a cell's cotangents are added to pbar once, when the
-// window leaves it. Neighbouring threads take neighbouring lines along the
+// cotangents, and a cell's cotangents go to pbar once, when the window
+// leaves it. The passes run in the order x, y, z: x stores into pbar, y into
+// pbarT, z adds to what x stored (and stores in the z halos, which x does not
+// reach), so no buffer is cleared first. Neighbouring threads take neighbouring lines along the
 // contiguous axis: y for the x and z faces in the reference layout, x for
 // the y faces, which run on the transposed copies.
 // Minimum resident blocks of the face kernel (its register budget).
@@ -757,7 +730,7 @@ __global__ void __launch_bounds__(256) vjp_prim_kernel(const VjpArgs a) {
 #endif
 
 template <typename T, int D, int SCHEME, int RIEMANN>
-__global__ void __launch_bounds__(128, SWC_VJP_FACE_MINB)
+__global__ void __launch_bounds__(kVjpFaceThreads, SWC_VJP_FACE_MINB)
     vjp_face_kernel(const VjpArgs a) {
   const int h = a.h;
   const int n = D == 0 ? a.nx : (D == 1 ? a.ny : a.nz);
@@ -773,7 +746,8 @@ __global__ void __launch_bounds__(128, SWC_VJP_FACE_MINB)
   const T hd = T(D == 0 ? a.dx : (D == 1 ? a.dy : a.dz));
   const T h1 = T(D == 0 ? a.dy : a.dx);
   const T h2 = T(D == 2 ? a.dy : a.dz);
-  const int nseg = (n + 1 + a.seg - 1) / a.seg;
+  const int seg = a.seg[D];
+  const int nseg = (n + seg) / seg;  // n + 1 faces
   // Thread index: the transverse coordinate along the contiguous axis
   // varies fastest (coalesced loads and atomics).
   const long long tid = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -792,8 +766,8 @@ __global__ void __launch_bounds__(128, SWC_VJP_FACE_MINB)
     }
     sg = (int)r;
   }
-  const int i0 = active ? sg * a.seg : 0;
-  const int i1 = active ? min(i0 + a.seg, n + 1) : 0;
+  const int i0 = active ? sg * seg : 0;
+  const int i1 = active ? min(i0 + seg, n + 1) : 0;
   const long long base = (long long)(c1 + h) * s1 + (long long)(c2 + h) * s2;
   const int vel[3] = {1 + D, D == 0 ? 2 : 1, D == 2 ? 2 : 3};
   const T* P[7];
@@ -827,20 +801,23 @@ __global__ void __launch_bounds__(128, SWC_VJP_FACE_MINB)
   };
   // A thread flushes cells i0-3 .. i1+1 of its line, each once. The five
   // head cells i0-3 .. i0+1 are also flushed by the previous segment's
-  // thread (they are its tail): this thread's part goes to hb, which the
-  // fix-up kernel adds. Every other cell gets exactly one addition in this
-  // pass, so the atomic below adds to a value no other thread changes
-  // meanwhile and the sum is the same on every run.
+  // thread (they are its tail): this thread's part goes to hb, which
+  // vjp_cell_kernel adds. Every other cell is written by one thread of this
+  // pass, so the z pass's atomic below adds to a value no other thread
+  // changes meanwhile and the sum is the same on every run.
   auto flush = [&](int j, const V2* b, T bh) {
     const long long o = base + (long long)(j + h) * st;
     const T val[7] = {b[0].x, b[1].x, b[1].y, b[2].x, b[0].y, b[2].y, bh};
     const int var[7] = {0, vel[0], vel[1], vel[2], 4, 5, 6};
-    if (j <= i0 + 1) {
+    if (j <= i0 + 1 && i0 > 0) {
 #pragma unroll
       for (int k = 0; k < 7; ++k) static_cast<T*>(a.hb[D][var[k]])[o] = val[k];
-    } else {
+    } else if (D == 2 && j >= 0 && j < n) {
 #pragma unroll
       for (int k = 0; k < 7; ++k) atomicAdd(static_cast<T*>(PBAR[var[k]]) + o, val[k]);
+    } else {
+#pragma unroll
+      for (int k = 0; k < 7; ++k) static_cast<T*>(PBAR[var[k]])[o] = val[k];
     }
   };
   // Window at face i (between cells i-1 and i): primitives sw[k] of cells
@@ -885,8 +862,8 @@ __global__ void __launch_bounds__(128, SWC_VJP_FACE_MINB)
   // velocity t1 and the normal velocity along t1, velocity t2 and the normal
   // velocity along t2). Their cotangents are stored per cell (tg; the head
   // cell i0-1 of a segment, whose face i0-1 belongs to the previous
-  // segment, into tgh) and moved onto the four neighbours by the fix-up
-  // kernel, which gathers them per target cell in a fixed order.
+  // segment, into tgh) and moved onto the four neighbours by
+  // vjp_cell_kernel, which gathers them per target cell in a fixed order.
   auto tang = [&](long long o, T* g4) {
     g4[0] = (P[vel[1]][o + s1] - P[vel[1]][o - s1]) * i2t1;
     g4[1] = (P[vel[0]][o + s1] - P[vel[0]][o - s1]) * i2t1;
@@ -901,7 +878,8 @@ __global__ void __launch_bounds__(128, SWC_VJP_FACE_MINB)
   // Tangential differences of cell i-1 and their cotangent so far.
   T g4a[4] = {T(0), T(0), T(0), T(0)}, gba[4] = {T(0), T(0), T(0), T(0)};
   if (a.visc && active) tang(base + (long long)(i0 - 1 + h) * st, g4a);
-  T nub = T(0);
+  // In double precision: a segment may hold any number of faces.
+  double nub = 0.0;
   for (int i = i0; i < i1; ++i) {
     load(i + 2, sw[5], swh[5]);
     if (i + 1 < i1) {
@@ -1081,7 +1059,7 @@ __global__ void __launch_bounds__(128, SWC_VJP_FACE_MINB)
     // One partial per block (a fixed shuffle tree per warp, the warps in
     // order), summed in a fixed order by vjp_nu_kernel.
     __shared__ double wsum[32];
-    double m = double(nub);
+    double m = nub;
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1)
       m += __shfl_xor_sync(0xffffffffu, m, off);
@@ -1101,98 +1079,73 @@ __global__ void __launch_bounds__(128, SWC_VJP_FACE_MINB)
 // head parts of the segments (hb) and, viscous, the tangential-difference
 // cotangents of the four neighbouring source cells (tg, plus tgh where the
 // source is the head cell i0-1 of a segment), always in the same order.
-// vjp_fix_kernel calls it once per pass for each cell, so no two threads
+// vjp_cell_kernel calls it once per pass for each cell, so no two threads
 // write one sum and the result does not depend on scheduling.
 template <typename T, int D>
-__device__ __forceinline__ int pass_parts(const VjpArgs& a, int c1, int c2,
-                                          int j, long long o, T* acc) {
+__device__ __forceinline__ void pass_parts(const VjpArgs& a, int c1, int c2,
+                                           int j, long long o, T* acc) {
   const int n = D == 0 ? a.nx : (D == 1 ? a.ny : a.nz);
   const int n1 = D == 0 ? a.ny : a.nx;
   const int n2 = D == 2 ? a.ny : a.nz;
   const long long s1 = D == 2 ? a.sx : 1;
   const long long s2 = D == 0 ? a.sz : (D == 1 ? a.tsz : 1);
-  constexpr int seg = kVjpSeg;  // a.seg
-  const int nseg = (n + 1 + seg - 1) / seg;
+  const unsigned seg = a.seg[D];
+  const unsigned nseg = (n + seg) / seg;
   const bool in1 = c1 >= 0 && c1 < n1, in2 = c2 >= 0 && c2 < n2;
   const int vel[3] = {1 + D, D == 0 ? 2 : 1, D == 2 ? 2 : 3};
-  int mask = 0;
-  // Head cells of segment sg: sg*seg-3 .. sg*seg+1 (seg >= 5: disjoint).
-  if (in1 && in2 && j >= -3 && (j + 3) % seg <= 4 && (j + 3) / seg < nseg) {
+  // Head cells of segment sg > 0: sg*seg-3 .. sg*seg+1 (seg >= 5: disjoint).
+  if (in1 && in2 && j + 3 >= (int)seg) {
+    const unsigned sg = (unsigned)(j + 3) / seg;
+    if (sg < nseg && (unsigned)(j + 3) - sg * seg <= 4) {
 #pragma unroll
-    for (int v = 0; v < 7; ++v) acc[v] += static_cast<const T*>(a.hb[D][v])[o];
-    mask = 0x7f;
+      for (int v = 0; v < 7; ++v)
+        acc[v] += __ldg(static_cast<const T*>(a.hb[D][v]) + o);
+    }
   }
-  if (!a.visc || j < -1 || j > n || !(in1 || in2) || c1 < -1 || c1 > n1 ||
-      c2 < -1 || c2 > n2)
-    return mask;
-  // Cotangent k of the tangential differences of source cell
-  // (j, c1+d1, c2+d2): its tg value (cells 0 .. n of a line) plus its tgh
-  // value where it is the head cell i0-1 of a segment.
-  const bool hj = (j + 1) % seg == 0 && (j + 1) / seg < nseg;
-  auto src = [&](int k, int d1, int d2) -> T {
-    const int e1 = c1 + d1, e2 = c2 + d2;
-    if (e1 < 0 || e1 >= n1 || e2 < 0 || e2 >= n2) return T(0);
-    const long long q = o + d1 * s1 + d2 * s2;
-    T v = j >= 0 ? static_cast<const T*>(a.tg[D][k])[q] : T(0);
-    if (hj) v += static_cast<const T*>(a.tgh[D][k])[q];
-    return v;
+  if (!a.visc || j < -1 || j > n) return;
+  // Cotangents k of the tangential differences of the source cells one step
+  // below (m) and above (p) along t1 and t2: the tg value (cells 0 .. n of a
+  // line) plus the tgh value where the source is the head cell i0-1 of a
+  // segment. Sources outside the lines count 0; their loads go to the cell
+  // itself, so that all of them are issued together.
+  const bool m1 = in2 && c1 >= 1 && c1 <= n1, p1 = in2 && c1 >= -1 && c1 < n1 - 1;
+  const bool m2 = in1 && c2 >= 1 && c2 <= n2, p2 = in1 && c2 >= -1 && c2 < n2 - 1;
+  const long long q1m = m1 ? o - s1 : o, q1p = p1 ? o + s1 : o;
+  const long long q2m = m2 ? o - s2 : o, q2p = p2 ? o + s2 : o;
+  T v[8];
+  auto load = [&](void* const* g, T* d) {
+    d[0] = __ldg(static_cast<const T*>(g[0]) + q1m);
+    d[1] = __ldg(static_cast<const T*>(g[0]) + q1p);
+    d[2] = __ldg(static_cast<const T*>(g[1]) + q1m);
+    d[3] = __ldg(static_cast<const T*>(g[1]) + q1p);
+    d[4] = __ldg(static_cast<const T*>(g[2]) + q2m);
+    d[5] = __ldg(static_cast<const T*>(g[2]) + q2p);
+    d[6] = __ldg(static_cast<const T*>(g[3]) + q2m);
+    d[7] = __ldg(static_cast<const T*>(g[3]) + q2p);
   };
+#pragma unroll
+  for (int k = 0; k < 8; ++k) v[k] = T(0);
+  if (j >= 0) load(a.tg[D], v);
+  const unsigned hs = (unsigned)(j + 1) / seg;
+  if (hs * seg == (unsigned)(j + 1) && hs < nseg) {
+    T w[8];
+    load(a.tgh[D], w);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] += w[k];
+  }
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const bool ok = k < 4 ? (k & 1 ? p1 : m1) : (k & 1 ? p2 : m2);
+    if (!ok) v[k] = T(0);
+  }
   const T h1 = T(D == 0 ? a.dy : a.dx);
   const T h2 = T(D == 2 ? a.dy : a.dz);
   const T i2t1 = T(1) / (T(2) * h1), i2t2 = T(1) / (T(2) * h2);
   // A source adds +g/(2 h_t) to its upper and -g/(2 h_t) to its lower
   // neighbour along t.
-  acc[vel[1]] += (src(0, -1, 0) - src(0, 1, 0)) * i2t1;
-  acc[vel[0]] += (src(1, -1, 0) - src(1, 1, 0)) * i2t1 +
-                 (src(3, 0, -1) - src(3, 0, 1)) * i2t2;
-  acc[vel[2]] += (src(2, 0, -1) - src(2, 0, 1)) * i2t2;
-  return mask | (1 << vel[0]) | (1 << vel[1]) | (1 << vel[2]);
-}
-
-// The face passes' parts outside pbar / pbarT (pass_parts), one thread per
-// cell of the padded grid: L = 0 adds the x and z passes' parts to pbar
-// (reference layout), L = 1 the y pass's to pbarT (transposed layout). No
-// two threads write one cell.
-template <typename T, int L>
-__global__ void __launch_bounds__(256) vjp_fix_kernel(const VjpArgs a) {
-  const int h = a.h;
-  const unsigned nxa = a.nx + 2 * h, nya = a.ny + 2 * h, nza = a.nz + 2 * h;
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (t >= (long long)nxa * nya * nza) return;
-  // 32-bit division: the host keeps the padded grid below 2^32 cells.
-  const unsigned tt = (unsigned)t;
-  T acc[7] = {T(0), T(0), T(0), T(0), T(0), T(0), T(0)};
-  int mask;
-  long long o;
-  void* const* PB;
-  if (L == 0) {  // (y fastest, x, z)
-    const unsigned q = tt / nya;
-    const int ya = (int)(tt - q * nya);
-    const int za = (int)(q / nxa);
-    const int xa = (int)(q - (unsigned)za * nxa);
-    o = za * a.sz + xa * a.sx + ya;
-    mask = pass_parts<T, 0>(a, ya - h, za - h, xa - h, o, acc);
-    mask |= pass_parts<T, 2>(a, xa - h, ya - h, za - h, o, acc);
-    PB = a.pbar;
-  } else {  // transposed: (x fastest, y, z)
-    const unsigned q = tt / nxa;
-    const int xt = (int)(tt - q * nxa);
-    const int za = (int)(q / nya);
-    const int yt = (int)(q - (unsigned)za * nya);
-    o = za * a.tsz + yt * a.tsy + xt;
-    mask = pass_parts<T, 1>(a, xt - h, za - h, yt - h, o, acc);
-    PB = a.pbarT;
-  }
-  if (!mask) return;
-  // Every load before any store (the compiler cannot tell PB from the
-  // arrays read above, and a load after a store would wait for it).
-  T cur[7];
-#pragma unroll
-  for (int v = 0; v < 7; ++v)
-    cur[v] = (mask >> v) & 1 ? static_cast<const T*>(PB[v])[o] : T(0);
-#pragma unroll
-  for (int v = 0; v < 7; ++v)
-    if ((mask >> v) & 1) static_cast<T*>(PB[v])[o] = cur[v] + acc[v];
+  acc[vel[1]] += (v[0] - v[1]) * i2t1;
+  acc[vel[0]] += (v[2] - v[3]) * i2t1 + (v[6] - v[7]) * i2t2;
+  acc[vel[2]] += (v[4] - v[5]) * i2t2;
 }
 
 // nu_bar += the per-warp partials of the three face passes, summed in a
@@ -1213,72 +1166,74 @@ __global__ void __launch_bounds__(256) vjp_nu_kernel(const double* part,
 }
 
 // Conserved cotangents of every cell from its primitive cotangents (the
-// reverse of cons_to_prim), plus the gravity source rho*G*g. The y faces'
-// cotangents are read back from the transposed layout through a tile.
-// Two resident blocks per SM in single precision (128 registers, 8 bytes
-// spilled: 1.7 % off the checkpointed KH 128^3 sweep, same gradient bits);
-// double precision needs ~250 registers and keeps one.
+// reverse of cons_to_prim), plus the gravity source rho*G*g. The primitive
+// cotangents are what the face passes stored and their parts outside pbar and
+// pbarT (pass_parts), summed here as they are read: two kernels that added
+// them to pbar and pbarT first moved 28 arrays more. The y faces' cotangents
+// come from the transposed layout through a tile. Memory bound; a thread
+// takes its four cells one after the other, so that three blocks fit on an SM
+// in single precision.
 template <typename T>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1) vjp_cell_kernel(const VjpArgs a) {
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 1) vjp_cell_kernel(const VjpArgs a) {
   T(*tiles)[TT][TT + 1] = vjp_tiles<T>();  // as in vjp_prim_kernel
-  const int nxa = a.nx + 2 * a.h, nya = a.ny + 2 * a.h;
+  const int h = a.h;
+  const int nxa = a.nx + 2 * h, nya = a.ny + 2 * h;
   const int za = blockIdx.z;
   const int y0 = blockIdx.x * TT, x0 = blockIdx.y * TT;
   const int tx = threadIdx.x, ty = threadIdx.y;
   const T gm1 = K<T>::gm1();
-  // Loads first (see vjp_prim_kernel): the cotangents of both layouts and
-  // the state, then the y faces' cotangents through the tile, then lam and
-  // the caller's terms.
-  T pbs[4][7], pbt[4][7], c4[4][5];
+  // Interior along an axis, and cells a pass along it writes (its faces'
+  // stencils reach three cells beyond).
+  auto in = [h](int c, int n) { return c >= h && c < n + h; };
+  auto reach = [h](int c, int n) { return c >= h - 3 && c < n + h + 3; };
+  const bool zin = in(za, a.nz), zre = reach(za, a.nz);
+  // The y faces' cotangents: tiles[v][y - y0][x - x0], written along x, read
+  // along y.
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    const int xa = x0 + ty + 8 * k, ya = y0 + tx;
-    const bool in = xa < nxa && ya < nya;
-    const long long o = za * a.sz + xa * a.sx + ya;
     const int xt = x0 + tx, yt = y0 + ty + 8 * k;
-    const bool int_ = xt < nxa && yt < nya;
-    const long long ot = za * a.tsz + yt * a.tsy + xt;
+    T t[7] = {T(0), T(0), T(0), T(0), T(0), T(0), T(0)};
+    if (xt < nxa && yt < nya) {
+      const long long o = za * a.tsz + yt * a.tsy + xt;
+      T acc[7] = {T(0), T(0), T(0), T(0), T(0), T(0), T(0)};
+      pass_parts<T, 1>(a, xt - h, za - h, yt - h, o, acc);
+      const bool st = zin && in(xt, a.nx) && reach(yt, a.ny);
 #pragma unroll
-    for (int v = 0; v < 7; ++v) {
-      pbs[k][v] = in ? static_cast<const T*>(a.pbar[v])[o] : T(0);
-      pbt[k][v] = int_ ? static_cast<const T*>(a.pbarT[v])[ot] : T(0);
+      for (int v = 0; v < 7; ++v)
+        t[v] = (st ? __ldg(static_cast<const T*>(a.pbarT[v]) + o) : T(0)) + acc[v];
     }
 #pragma unroll
-    for (int v = 0; v < 5; ++v)
-      c4[k][v] = in ? static_cast<const T*>(a.uk[v])[o] : T(1);
-  }
-  // tiles[v][y - y0][x - x0], written along x, read along y.
-#pragma unroll
-  for (int v = 0; v < kCellTiles; ++v) {
-#pragma unroll
-    for (int k = 0; k < 4; ++k) tiles[v][ty + 8 * k][tx] = pbt[k][v];
+    for (int v = 0; v < kCellTiles; ++v) tiles[v][ty + 8 * k][tx] = t[v];
   }
   __syncthreads();
-#pragma unroll
-  for (int v = 0; v < kCellTiles; ++v) {
-#pragma unroll
-    for (int k = 0; k < 4; ++k) pbs[k][v] += tiles[v][tx][ty + 8 * k];
-  }
-  T l4[4][5], x14[4][5], x24[4][5];
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const int xa = x0 + ty + 8 * k, ya = y0 + tx;
-    const bool in = xa < nxa && ya < nya;
-    const long long o = za * a.sz + xa * a.sx + ya;
-#pragma unroll
-    for (int v = 0; v < 5; ++v) {
-      l4[k][v] = in ? static_cast<const T*>(a.lam[v])[o] : T(0);
-      x14[k][v] = in && a.x1[v] ? static_cast<const T*>(a.x1[v])[o] : T(0);
-      x24[k][v] = in && a.x2[v] ? static_cast<const T*>(a.x2[v])[o] : T(0);
-    }
-  }
-#pragma unroll
+#pragma unroll 1
   for (int k = 0; k < 4; ++k) {
     const int xa = x0 + ty + 8 * k, ya = y0 + tx;
     if (xa >= nxa || ya >= nya) continue;
     const long long o = za * a.sz + xa * a.sx + ya;
-    const T* c = c4[k];
-    const T* pb = pbs[k];
+    const bool xin = in(xa, a.nx), yin = in(ya, a.ny);
+    const bool interior = xin && yin && zin;
+    T c[5], l[5], x1[5], x2[5], pb[7];
+#pragma unroll
+    for (int v = 0; v < 5; ++v) {
+      c[v] = __ldg(static_cast<const T*>(a.uk[v]) + o);
+      l[v] = interior ? __ldg(static_cast<const T*>(a.lam[v]) + o) : T(0);
+      x1[v] = interior && a.x1[v] ? __ldg(static_cast<const T*>(a.x1[v]) + o) : T(0);
+      x2[v] = interior && a.x2[v] ? __ldg(static_cast<const T*>(a.x2[v]) + o) : T(0);
+    }
+    {
+      // Written by the x pass, the z pass or both.
+      const bool st = yin && ((zin && reach(xa, a.nx)) || (xin && zre));
+      T acc[7] = {T(0), T(0), T(0), T(0), T(0), T(0), T(0)};
+#pragma unroll
+      for (int v = 0; v < 7; ++v)
+        pb[v] = st ? __ldg(static_cast<const T*>(a.pbar[v]) + o) : T(0);
+      pass_parts<T, 0>(a, ya - h, za - h, xa - h, o, acc);
+      pass_parts<T, 2>(a, xa - h, ya - h, za - h, o, acc);
+#pragma unroll
+      for (int v = 0; v < 7; ++v)
+        pb[v] = (pb[v] + acc[v]) + tiles[v][tx][ty + 8 * k];
+    }
     const T pe = pe_of<T>(a, xa, ya, za);
     const T rho = c[0];
     const T inv = T(1) / rho;
@@ -1309,13 +1264,11 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1) vjp_cell_kernel(c
     }
     rb += -invb * inv * inv;
     // Gravity source on the momenta of interior cells.
-    const bool interior = xa >= a.h && xa < a.nx + a.h && ya >= a.h &&
-                          ya < a.ny + a.h && za >= a.h && za < a.nz + a.h;
     if (a.gravity_mask && interior) {
 #pragma unroll
       for (int d = 0; d < 3; ++d)
         if (a.gravity_mask & (1 << d))
-          rb += T(a.beta) * l4[k][1 + d] * K<T>::grav() * T(a.g[d]);
+          rb += T(a.beta) * l[1 + d] * K<T>::grav() * T(a.g[d]);
     }
     out[0] = rb;
     // The caller's combination on the interior (alpha*lam + c1*x1 + c2*x2):
@@ -1324,8 +1277,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1) vjp_cell_kernel(c
     if (interior) {
 #pragma unroll
       for (int v = 0; v < 5; ++v)
-        out[v] += T(a.alpha) * l4[k][v] + T(a.c1) * x14[k][v] +
-                  T(a.c2) * x24[k][v];
+        out[v] += T(a.alpha) * l[v] + T(a.c1) * x1[v] + T(a.c2) * x2[v];
     }
 #pragma unroll
     for (int v = 0; v < 5; ++v) static_cast<T*>(a.vout[v])[o] = out[v];
@@ -1440,6 +1392,32 @@ __global__ void __launch_bounds__(256) vjp_halo_kernel(const VjpHalo a,
   }
 }
 
+// Faces per thread of a face pass over `lines` lines of `faces` faces. Two
+// blocks fit on an SM (255 registers); a thread's time is about its faces and
+// two more (its window's first cells and its last cell's reverse), and the
+// pass takes ceil(blocks / slots) rounds of them: the count that minimises
+// rounds x (seg + 2), the longest of equals (fewer heads). At 96^3 that is
+// one round of four segments of 25 faces; with 16 everywhere it was two
+// rounds and a seventh segment of one face.
+int face_seg(int faces, long long lines) {
+  const long long slots = 2LL * sm_count();
+  long long least = -1;
+  int best = faces;
+  for (int nseg = 1; nseg <= faces; ++nseg) {
+    const int seg = (faces + nseg - 1) / nseg;
+    if (seg < kVjpMinSeg && nseg > 1) break;
+    const long long used = (faces + seg - 1) / seg;
+    const long long blocks =
+        (lines * used + kVjpFaceThreads - 1) / kVjpFaceThreads;
+    const long long cost = (blocks + slots - 1) / slots * (seg + 2);
+    if (least < 0 || cost < least) {
+      least = cost;
+      best = seg;
+    }
+  }
+  return best;
+}
+
 // Above 48 KB of dynamic shared memory a kernel must opt in: done on the
 // first call per dtype (whatever the scheme), which the header asks callers
 // to make outside stream capture.
@@ -1470,7 +1448,7 @@ int launch_vjp(const VjpArgs& a, const SwcFieldBC* bcs, cudaStream_t s) {
   vjp_prim_kernel<T><<<tgrid, tblock, kPrimTiles * tile_bytes, s>>>(a);
   note_launch();
   // Face passes; the blocks' nu partials of pass D start at nu_off[D].
-  const int ft = 128;
+  const int ft = kVjpFaceThreads;
   VjpArgs b = a;
   unsigned blocks[3];
   long long parts = 0;
@@ -1478,7 +1456,7 @@ int launch_vjp(const VjpArgs& a, const SwcFieldBC* bcs, cudaStream_t s) {
     const int n = D == 0 ? a.nx : (D == 1 ? a.ny : a.nz);
     const int n1 = D == 0 ? a.ny : a.nx;
     const int n2 = D == 2 ? a.ny : a.nz;
-    const long long nseg = (n + 1 + a.seg - 1) / a.seg;
+    const long long nseg = (n + a.seg[D]) / a.seg[D];
     const long long threads = (long long)n1 * n2 * nseg;
     blocks[D] = (unsigned)((threads + ft - 1) / ft);
     b.nu_off[D] = parts;
@@ -1488,14 +1466,6 @@ int launch_vjp(const VjpArgs& a, const SwcFieldBC* bcs, cudaStream_t s) {
     if (D == 0) vjp_face_kernel<T, 0, SCHEME, RIEMANN><<<blocks[D], ft, 0, s>>>(b);
     else if (D == 1) vjp_face_kernel<T, 1, SCHEME, RIEMANN><<<blocks[D], ft, 0, s>>>(b);
     else vjp_face_kernel<T, 2, SCHEME, RIEMANN><<<blocks[D], ft, 0, s>>>(b);
-    note_launch();
-  }
-  {
-    const long long cells = (long long)nxa * nya * nza;
-    const unsigned fb = (unsigned)((cells + 255) / 256);
-    vjp_fix_kernel<T, 0><<<fb, 256, 0, s>>>(b);
-    note_launch();
-    vjp_fix_kernel<T, 1><<<fb, 256, 0, s>>>(b);
     note_launch();
   }
   if (b.visc && b.nu_bar) {
@@ -1699,10 +1669,10 @@ int stage_vjp(const SwcGrid* grid, const SwcScheme* sc, const SwcFieldBC* bcs,
     const int nd[3] = {grid->nx, grid->ny, grid->nz};
     for (int D = 0; D < 3; ++D) {
       const long long n1 = nd[D == 0 ? 1 : 0], n2 = nd[D == 2 ? 1 : 2];
-      const long long threads = n1 * n2 * ((nd[D] + 1 + kVjpSeg - 1) / kVjpSeg);
-      parts += (threads + 127) / 128;
-      // Columns of the halo reverse and cells of the fix-up (32-bit index
-      // arithmetic).
+      a.seg[D] = face_seg(nd[D] + 1, n1 * n2);
+      const long long threads = n1 * n2 * ((nd[D] + a.seg[D]) / a.seg[D]);
+      parts += (threads + kVjpFaceThreads - 1) / kVjpFaceThreads;
+      // Columns of the halo reverse (32-bit index arithmetic).
       most = std::max(most, a.tsz * (long long)(grid->nz + 2 * grid->halo));
       most = std::max(most, 5LL * (n1 + 2LL * grid->halo) *
                                 (n2 + 2LL * grid->halo));
@@ -1725,7 +1695,6 @@ int stage_vjp(const SwcGrid* grid, const SwcScheme* sc, const SwcFieldBC* bcs,
   a.beta = beta;
   a.gravity_mask = sc->gravity_mask;
   a.nu_bar = nu_bar;
-  a.seg = kVjpSeg;
   a.limiter = sc->limiter;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const bool f32 = sc->dtype == SWC_F32;

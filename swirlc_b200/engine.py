@@ -369,6 +369,18 @@ class Solver:
         ctypes.byref(self.grid), self.scheme.dtype, len(fields), ptrs,
         self.bcs, 0, nat.stream_ptr()), 'halo fill')
 
+  def copy_filled(self, fields: Sequence[torch.Tensor],
+                  out: Sequence[torch.Tensor]) -> None:
+    """out = copies of `fields` with their halos filled (one pass)."""
+    if self._layout is not None:
+      for a, b in zip(out, fields):
+        a.copy_(b)
+      self.fill_halos(out)
+      return
+    nat.check(nat.load().swc_halo_copy(
+        self.grid, self.scheme.dtype, len(fields), nat.ptr_array(fields),
+        nat.ptr_array(out), None, self.bcs, 0, nat.stream_ptr()), 'halo copy')
+
   def fill_boundary_dim(self, fields: Sequence[torch.Tensor], dim: int) -> None:
     """Halo fill along `dim` of the sides that take a boundary condition
     (not the sides shared with another replica)."""
