@@ -200,8 +200,9 @@ int launch_halo(const HaloBatch& b, cudaStream_t s) {
 // swc_halo_fill does for one grid with rho at index 0.
 int batch_halo(const std::vector<Plan>& plans, int set, int dtype,
                cudaStream_t s) {
-  // Members whose halos take one pass go through shell_batch_kernel; the
-  // others through the x, y, z passes below.
+  // Members whose halos take one pass go through shell_batch_kernel, or need
+  // none where a stage reads a work state's halos from the interior
+  // (batch_stage); the others through the x, y, z passes below.
   std::vector<char> shell(plans.size(), 0);
   {
     ShellBatch sb;
@@ -211,6 +212,7 @@ int batch_halo(const std::vector<Plan>& plans, int set, int dtype,
       int clamp[3];
       if (!shell_ok(m, clamp)) continue;
       shell[i] = 1;
+      if (set > 0) continue;
       ShellMember& sm = sb.m[sb.n];
       memset(&sm, 0, sizeof(sm));
       sm.g.nf = 5;
@@ -362,7 +364,7 @@ int batch_stage(const std::vector<Plan>& plans, const SwcScheme* sc, int in,
         a.u0[v] = mode >= SWC_OUT_CONVEX ? m.u[v] : nullptr;
         a.uout[v] = field_of(m, out, v);
       }
-      a.mode = mode; a.c0 = c0; a.c1 = c1;
+      stage_weights(a, mode, c0, c1);
       a.dt = &m.clock->dt;
       a.dtmin_out = reduce ? &m.clock->dtmin : nullptr;
       for (int d = 0; d < 3; ++d) {
@@ -374,6 +376,10 @@ int batch_stage(const std::vector<Plan>& plans, const SwcScheme* sc, int in,
       a.nu = sc->nu; a.pr = sc->pr > 0 ? sc->pr : 1.0;
       a.gravity_mask = sc->gravity_mask;
       a.zseg = p.zseg;
+      int clamp[3];
+      if (in > 0 && shell_ok(m, clamp))
+        for (int d = 0; d < 3; ++d)
+          a.halo_from[d] = clamp[d] ? kHaloClamped : kHaloWrapped;
       b.pre[b.n + 1] = b.pre[b.n] + p.ctas;
       if (++b.n == SWC_BATCH_CHUNK) {
         const int rc = launch_stage_group(sc, b, tile, s);

@@ -77,24 +77,23 @@ __global__ void halo_kernel(const HaloArgs a) {
     halo_elem<T>(a, t);
 }
 
-// What a one-pass halo fill does to the device clock beside its own work, so
-// that a step needs no launches for it: the fill before the first stage
-// starts the step, the fill before the last one ends it (no kernel of the
-// step reads or writes t or the step count in between).
-enum ClockTick { kTickNone, kTickBegin, kTickEnd };
-__device__ __forceinline__ void clock_tick(SwcClock* c, int tick, int t) {
-  if (t != 0) return;
-  if (tick == kTickBegin) clock_begin(c);
-  if (tick == kTickEnd) clock_end(c);
+// A one-pass halo fill also advances the device clock of the step it starts
+// (clock not NULL), so that the step needs no launches for it: dt is chosen,
+// then t and the step count move on, which no kernel of the step reads.
+__device__ __forceinline__ void clock_tick(SwcClock* c, int t) {
+  if (!c || t != 0) return;
+  clock_begin(c);
+  clock_end(c);
 }
+__global__ void clock_tick_kernel(SwcClock* c) { clock_tick(c, 0); }
 
 // One-pass halo fill of one grid (halo_shell_elem, swc_halo.cuh).
 template <typename T>
 __global__ void halo_periodic_kernel(const HaloArgs a, int total,
                                      int clamp_x, int clamp_y, int clamp_z,
-                                     SwcClock* clock, int tick) {
+                                     SwcClock* clock) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  clock_tick(clock, tick, t);
+  clock_tick(clock, t);
   if (t < total) halo_shell_elem<T>(a, t, clamp_x, clamp_y, clamp_z);
 }
 
@@ -102,10 +101,15 @@ __global__ void halo_periodic_kernel(const HaloArgs a, int total,
 // (halo_shell_bc_elem, swc_halo.cuh).
 template <typename T>
 __global__ void halo_shell_kernel(const ShellArgs a, int total,
-                                  SwcClock* clock, int tick) {
+                                  SwcClock* clock) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  clock_tick(clock, tick, t);
+  clock_tick(clock, t);
   if (t < total) halo_shell_bc_elem<T>(a, t);
+}
+template <typename T>
+__global__ void halo_clear_kernel(const ShellArgs a, int total) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < total) halo_clear_elem<T>(a, t);
 }
 
 // Copy of every field with its halos filled (halo_copy_elem, swc_halo.cuh):
@@ -593,11 +597,33 @@ static bool shell_args(const SwcGrid* grid, int nfields,
           b[0].value == 0.0 && b[1].value == 0.0)
         ++clamp;
     }
-    sa.dims[d] = wrap == nfields ? kShellWrap
-                                 : clamp == nfields ? kShellClamp : kShellMixed;
+    sa.dims[d] = wrap == nfields ? kHaloWrapped
+                                 : clamp == nfields ? kHaloClamped : kHaloStored;
   }
   sa.nx = grid->nx; sa.ny = grid->ny; sa.nz = grid->nz; sa.h = h;
   sa.sx = grid->sx; sa.sz = grid->sz;
+  return true;
+}
+
+// Where a stage may read halo cells of fields with conditions `bcs` from
+// (StageArgs::halo_from), so that they need no fill before it: possible where
+// every dim has one source for all fields. Two fills of an RK3 step and the
+// copy of a functional call go this way (each 3 to 4 us of a small step's 40,
+// 23 us of 1.49 ms at 256^3). `none`: all stored.
+struct HaloFrom {
+  int d[3];
+};
+static const HaloFrom kAllStored = {{kHaloStored, kHaloStored, kHaloStored}};
+static bool halo_from_interior(const SwcGrid* grid, int nfields,
+                               const void* const* fields,
+                               const SwcFieldBC* bcs, bool any_prim,
+                               HaloFrom* from) {
+  *from = kAllStored;
+  ShellArgs sa;
+  if (!shell_args(grid, nfields, fields, bcs, any_prim, sa)) return false;
+  for (int d = 0; d < 3; ++d)
+    if (sa.dims[d] == kHaloStored) return false;
+  for (int d = 0; d < 3; ++d) from->d[d] = sa.dims[d];
   return true;
 }
 
@@ -605,8 +631,7 @@ static bool shell_args(const SwcGrid* grid, int nfields,
 // pass, else in a launch of its own.
 static int halo_fill(const SwcGrid* grid, int32_t dtype, int32_t nfields,
                      void* const* fields, const SwcFieldBC* bcs,
-                     int32_t rho_index, SwcClock* clock, int tick,
-                     void* stream) {
+                     int32_t rho_index, SwcClock* clock, void* stream) {
   swc::NvtxRange nvtx_range_("swc_halo_fill");
   bool any_prim = false;
   int st = check_halo(grid, dtype, nfields, fields, bcs, rho_index, &any_prim);
@@ -648,10 +673,10 @@ static int halo_fill(const SwcGrid* grid, int32_t dtype, int32_t nfields,
       const unsigned blocks = (unsigned)((total + threads - 1) / threads);
       if (dtype == SWC_F32)
         halo_periodic_kernel<float><<<blocks, threads, 0, s>>>(
-            a, (int)total, clamp[0], clamp[1], clamp[2], clock, tick);
+            a, (int)total, clamp[0], clamp[1], clamp[2], clock);
       else
         halo_periodic_kernel<double><<<blocks, threads, 0, s>>>(
-            a, (int)total, clamp[0], clamp[1], clamp[2], clock, tick);
+            a, (int)total, clamp[0], clamp[1], clamp[2], clock);
       note_launch();
       return check_launch("halo_fill");
     }
@@ -663,16 +688,19 @@ static int halo_fill(const SwcGrid* grid, int32_t dtype, int32_t nfields,
       const unsigned blocks = (unsigned)((total + threads - 1) / threads);
       if (dtype == SWC_F32)
         halo_shell_kernel<float><<<blocks, threads, 0, s>>>(sa, (int)total,
-                                                            clock, tick);
+                                                            clock);
       else
         halo_shell_kernel<double><<<blocks, threads, 0, s>>>(sa, (int)total,
-                                                             clock, tick);
+                                                             clock);
       note_launch();
       return check_launch("halo_fill");
     }
   }
-  if (tick == kTickBegin && (st = swc_clock_begin_step(clock, stream))) return st;
-  if (tick == kTickEnd && (st = swc_clock_end_step(clock, stream))) return st;
+  if (clock) {
+    clock_tick_kernel<<<1, 1, 0, s>>>(clock);
+    note_launch();
+    if ((st = check_launch("clock"))) return st;
+  }
   if (h == 0) return SWC_OK;
   // Phase 0: fields with direct BCs; phase 1: fields with primitive BCs,
   // after rho is complete in all three dims.
@@ -721,7 +749,7 @@ int swc_halo_fill(const SwcGrid* grid, int32_t dtype, int32_t nfields,
                   void* const* fields, const SwcFieldBC* bcs,
                   int32_t rho_index, void* stream) {
   return halo_fill(grid, dtype, nfields, fields, bcs, rho_index, nullptr,
-                   kTickNone, stream);
+                   stream);
 }
 
 int swc_halo_copy(const SwcGrid* grid, int32_t dtype, int32_t nfields,
@@ -781,7 +809,8 @@ int swc_halo_copy(const SwcGrid* grid, int32_t dtype, int32_t nfields,
 static int stage_args(const SwcGrid* grid, const SwcScheme* sc, int nf,
                       const void* const* uk, const void* const* u0,
                       void* const* uout, int32_t mode, double c0, double c1,
-                      const double* dt, double* dtmin_out, StageArgs& a) {
+                      const double* dt, double* dtmin_out,
+                      const HaloFrom& from, StageArgs& a) {
   int st = check_grid(grid);
   if (st) return st;
   if (!sc) return fail(SWC_ERR_ARG, "scheme is NULL");
@@ -814,7 +843,8 @@ static int stage_args(const SwcGrid* grid, const SwcScheme* sc, int nf,
     a.u0[v] = u0 ? u0[v] : nullptr;
     a.uout[v] = uout[v];
   }
-  a.mode = mode; a.c0 = c0; a.c1 = c1; a.dt = dt; a.dtmin_out = dtmin_out;
+  stage_weights(a, mode, c0, c1);
+  a.dt = dt; a.dtmin_out = dtmin_out;
   for (int d = 0; d < 3; ++d) {
     a.pe[d] = sc->pe_axis[d];
     if (sc->pe_axis[d]) a.has_pe = 1;
@@ -824,19 +854,22 @@ static int stage_args(const SwcGrid* grid, const SwcScheme* sc, int nf,
   a.nu = sc->nu; a.pr = sc->pr > 0 ? sc->pr : 1.0;
   a.gravity_mask = sc->gravity_mask;
   a.zseg = std::max(0, std::min(sc->zseg, grid->nz));
+  for (int d = 0; d < 3; ++d) a.halo_from[d] = from.d[d];
   return SWC_OK;
 }
 
-int swc_rk_stage(const SwcGrid* grid, const SwcScheme* sc,
-                 const void* const* uk, const void* const* u0,
-                 void* const* uout, int32_t mode, double c0, double c1,
-                 const double* dt, double* dtmin_out, void* stream) {
+static int plain_stage(const SwcGrid* grid, const SwcScheme* sc,
+                       const void* const* uk, const void* const* u0,
+                       void* const* uout, int32_t mode, double c0, double c1,
+                       const double* dt, double* dtmin_out,
+                       const HaloFrom& from, void* stream) {
   swc::NvtxRange nvtx_range_("swc_rk_stage");
   if (sc && sc->nscalars != 0)
     return fail(SWC_ERR_UNSUPPORTED,
                 "transported scalars go through swc_rk_stage_ext");
   StageArgs a;
-  int st = stage_args(grid, sc, 5, uk, u0, uout, mode, c0, c1, dt, dtmin_out, a);
+  int st = stage_args(grid, sc, 5, uk, u0, uout, mode, c0, c1, dt, dtmin_out,
+                      from, a);
   if (st) return st;
   const int visc = sc->diffusion ? 1 : 0;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
@@ -860,11 +893,19 @@ int swc_rk_stage(const SwcGrid* grid, const SwcScheme* sc,
   return SWC_OK;
 }
 
-int swc_rk_stage_ext(const SwcGrid* grid, const SwcScheme* sc,
+int swc_rk_stage(const SwcGrid* grid, const SwcScheme* sc,
+                 const void* const* uk, const void* const* u0,
+                 void* const* uout, int32_t mode, double c0, double c1,
+                 const double* dt, double* dtmin_out, void* stream) {
+  return plain_stage(grid, sc, uk, u0, uout, mode, c0, c1, dt, dtmin_out,
+                     kAllStored, stream);
+}
+
+static int ext_stage(const SwcGrid* grid, const SwcScheme* sc,
                      const SwcStageExt* ext, const void* const* uk,
                      const void* const* u0, void* const* uout, int32_t mode,
                      double c0, double c1, const double* dt,
-                     double* dtmin_out, void* stream) {
+                     double* dtmin_out, const HaloFrom& from, void* stream) {
   swc::NvtxRange nvtx_range_("swc_rk_stage_ext");
   if (!sc) return fail(SWC_ERR_ARG, "scheme is NULL");
   const int ns = sc->nscalars;
@@ -911,7 +952,7 @@ int swc_rk_stage_ext(const SwcGrid* grid, const SwcScheme* sc,
                 "enabled at this time.");
   StageArgs a;
   int st = stage_args(grid, sc, 5 + ns, uk, u0, uout, mode, c0, c1, dt,
-                      dtmin_out, a);
+                      dtmin_out, from, a);
   if (st) return st;
   const int visc = sc->diffusion ? 1 : 0;
   const int help = e.p_ref ? 1 : 0;
@@ -935,6 +976,15 @@ int swc_rk_stage_ext(const SwcGrid* grid, const SwcScheme* sc,
   }
   if (rc) return fail(rc, "stage launch failed: %s", cudaGetErrorString(cudaGetLastError()));
   return SWC_OK;
+}
+
+int swc_rk_stage_ext(const SwcGrid* grid, const SwcScheme* sc,
+                     const SwcStageExt* ext, const void* const* uk,
+                     const void* const* u0, void* const* uout, int32_t mode,
+                     double c0, double c1, const double* dt,
+                     double* dtmin_out, void* stream) {
+  return ext_stage(grid, sc, ext, uk, u0, uout, mode, c0, c1, dt, dtmin_out,
+                   kAllStored, stream);
 }
 
 int swc_cfl_reduce(const SwcGrid* grid, const SwcScheme* sc,
@@ -1216,11 +1266,12 @@ int swc_rk_combine(int64_t n, int32_t dtype, int32_t mode, double c0,
 static int run_stage(const SwcGrid* grid, const SwcScheme* scheme,
                      const SwcStageExt* ext, const void* const* uk,
                      const void* const* u0, void* const* uout, int32_t mode,
-                     double c0, double c1, const double* dt, void* stream) {
-  return ext ? swc_rk_stage_ext(grid, scheme, ext, uk, u0, uout, mode, c0, c1,
-                                dt, nullptr, stream)
-             : swc_rk_stage(grid, scheme, uk, u0, uout, mode, c0, c1, dt,
-                            nullptr, stream);
+                     double c0, double c1, const double* dt,
+                     const HaloFrom& from, void* stream) {
+  return ext ? ext_stage(grid, scheme, ext, uk, u0, uout, mode, c0, c1, dt,
+                         nullptr, from, stream)
+             : plain_stage(grid, scheme, uk, u0, uout, mode, c0, c1, dt,
+                           nullptr, from, stream);
 }
 
 int swc_rk_step(const SwcGrid* grid, const SwcScheme* scheme,
@@ -1246,34 +1297,47 @@ int swc_rk_step(const SwcGrid* grid, const SwcScheme* scheme,
   }
   const double* dt = &clock_dev->dt;
   double* dtmin = &clock_dev->dtmin;
-  if ((st = halo_fill(grid, scheme->dtype, 5, u, bcs, 0, clock_dev, kTickBegin,
-                      stream)))
+  if ((st = halo_fill(grid, scheme->dtype, 5, u, bcs, 0, clock_dev, stream)))
     return st;
-  if ((st = swc_rk_stage(grid, scheme, (const void* const*)u, nullptr, w1,
-                         SWC_OUT_EULER, 0.0, 0.0, dt, nullptr, stream)))
+  // The work states' halos are read from the interior where they can be.
+  bool any_prim = false;
+  for (int v = 0; v < 5; ++v) any_prim |= bcs[v].via_primitive != 0;
+  HaloFrom from;
+  const bool fill = !halo_from_interior(grid, 5, (const void* const*)u, bcs,
+                                        any_prim, &from);
+  const void* const* cu = (const void* const*)u;
+  if ((st = plain_stage(grid, scheme, cu, nullptr, w1, SWC_OUT_EULER, 0.0, 0.0,
+                        dt, nullptr, kAllStored, stream)))
     return st;
-  if ((st = halo_fill(grid, scheme->dtype, 5, w1, bcs, 0, clock_dev,
-                      order == 3 ? kTickNone : kTickEnd, stream)))
+  if (fill && (st = swc_halo_fill(grid, scheme->dtype, 5, w1, bcs, 0, stream)))
     return st;
-  if (order == 3) {
-    if ((st = swc_rk_stage(grid, scheme, (const void* const*)w1,
-                           (const void* const*)u, w2, SWC_OUT_CONVEX, 0.75,
-                           0.25, dt, nullptr, stream)))
-      return st;
-    if ((st = halo_fill(grid, scheme->dtype, 5, w2, bcs, 0, clock_dev, kTickEnd,
-                        stream)))
-      return st;
-    if ((st = swc_rk_stage(grid, scheme, (const void* const*)w2,
-                           (const void* const*)u, u, SWC_OUT_CONVEX,
-                           1.0 / 3.0, 2.0 / 3.0, dt, dtmin, stream)))
-      return st;
-  } else {
-    if ((st = swc_rk_stage(grid, scheme, (const void* const*)w1,
-                           (const void* const*)u, u, SWC_OUT_AVERAGE, 0.5, 0.0,
-                           dt, dtmin, stream)))
-      return st;
-  }
-  return SWC_OK;
+  if (order == 2)
+    return plain_stage(grid, scheme, (const void* const*)w1, cu, u,
+                       SWC_OUT_AVERAGE, 0.5, 0.0, dt, dtmin, from, stream);
+  if ((st = plain_stage(grid, scheme, (const void* const*)w1, cu, w2,
+                        SWC_OUT_CONVEX, 0.75, 0.25, dt, nullptr, from, stream)))
+    return st;
+  if (fill && (st = swc_halo_fill(grid, scheme->dtype, 5, w2, bcs, 0, stream)))
+    return st;
+  return plain_stage(grid, scheme, (const void* const*)w2, cu, u,
+                     SWC_OUT_CONVEX, 1.0 / 3.0, 2.0 / 3.0, dt, dtmin, from,
+                     stream);
+}
+
+// Where the first stage of a functional call may read the caller's fields as
+// they are: every dim with one source for all fields, and no reference state,
+// which is read at the halo cell itself.
+static int functional_source(const SwcGrid* grid, const SwcScheme* scheme,
+                             const SwcFieldBC* bcs, const SwcStageExt* ext,
+                             const void* const* u, bool* mapped,
+                             HaloFrom* from) {
+  bool any_prim = false;
+  const int nf = 5 + scheme->nscalars;
+  const int st = check_halo(grid, scheme->dtype, nf, u, bcs, 0, &any_prim);
+  *from = kAllStored;
+  *mapped = !st && !(ext && ext->p_ref) &&
+            halo_from_interior(grid, nf, u, bcs, any_prim, from);
+  return st;
 }
 
 int swc_rhs(const SwcGrid* grid, const SwcScheme* scheme,
@@ -1286,11 +1350,37 @@ int swc_rhs(const SwcGrid* grid, const SwcScheme* scheme,
   const int ns = scheme->nscalars;
   if (ns < 0 || ns > 3)
     return fail(SWC_ERR_UNSUPPORTED, "%d transported scalars (at most 3)", ns);
-  const int st = swc_halo_copy(grid, scheme->dtype, 5 + ns, u, work, out, bcs,
-                               0, stream);
+  bool mapped;
+  HaloFrom from;
+  int st = functional_source(grid, scheme, bcs, ext, u, &mapped, &from);
   if (st) return st;
-  return run_stage(grid, scheme, ext, (const void* const*)work, nullptr, out,
-                   SWC_OUT_RHS, 0.0, 0.0, nullptr, stream);
+  const long long total =
+      halo_shell_count(grid->nx, grid->ny, grid->nz, grid->halo);
+  if (!mapped || total >= (1LL << 31)) {
+    if ((st = swc_halo_copy(grid, scheme->dtype, 5 + ns, u, work, out, bcs, 0,
+                            stream)))
+      return st;
+    return run_stage(grid, scheme, ext, (const void* const*)work, nullptr, out,
+                     SWC_OUT_RHS, 0.0, 0.0, nullptr, kAllStored, stream);
+  }
+  if ((st = run_stage(grid, scheme, ext, u, nullptr, out, SWC_OUT_RHS, 0.0, 0.0,
+                      nullptr, from, stream)))
+    return st;
+  if (total == 0) return SWC_OK;
+  ShellArgs sa;
+  memset(&sa, 0, sizeof(sa));
+  sa.nf = 5 + ns;
+  for (int v = 0; v < sa.nf; ++v) sa.fld[v].f = out[v];
+  sa.nx = grid->nx; sa.ny = grid->ny; sa.nz = grid->nz; sa.h = grid->halo;
+  sa.sx = grid->sx; sa.sz = grid->sz;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const unsigned blocks = (unsigned)((total + 255) / 256);
+  if (scheme->dtype == SWC_F32)
+    halo_clear_kernel<float><<<blocks, 256, 0, s>>>(sa, (int)total);
+  else
+    halo_clear_kernel<double><<<blocks, 256, 0, s>>>(sa, (int)total);
+  note_launch();
+  return check_launch("rhs");
 }
 
 int swc_rk_step_out(const SwcGrid* grid, const SwcScheme* scheme,
@@ -1307,28 +1397,37 @@ int swc_rk_step_out(const SwcGrid* grid, const SwcScheme* scheme,
   if (ns < 0 || ns > 3)
     return fail(SWC_ERR_UNSUPPORTED, "%d transported scalars (at most 3)", ns);
   const int nf = 5 + ns;
-  // The filled input, and the stage state that is not `out`: RK3 passes
-  // through out, w, out; RK2 through w, out.
-  void* const* u0 = work;
+  bool mapped;
+  HaloFrom from;
+  int st = functional_source(grid, scheme, bcs, ext, u, &mapped, &from);
+  if (st) return st;
+  // The input (filled copy, unless its halos are read from the interior) and
+  // the stage state that is not `out`: RK3 passes through out, w, out; RK2
+  // through w, out.
   void* const* w = work + nf;
   void* const* first = order == 3 ? out : w;
-  int st = swc_halo_copy(grid, dtype, nf, u, u0, nullptr, bcs, 0, stream);
-  if (st) return st;
-  const void* const* cu0 = (const void* const*)u0;
+  const void* const* cu0 = u;
+  if (!mapped) {
+    if ((st = swc_halo_copy(grid, dtype, nf, u, work, nullptr, bcs, 0, stream)))
+      return st;
+    cu0 = (const void* const*)work;
+  }
   if ((st = run_stage(grid, scheme, ext, cu0, nullptr, first, SWC_OUT_EULER,
-                      0.0, 0.0, dt, stream)))
+                      0.0, 0.0, dt, from, stream)))
     return st;
-  if ((st = swc_halo_fill(grid, dtype, nf, first, bcs, 0, stream))) return st;
+  if (!mapped && (st = swc_halo_fill(grid, dtype, nf, first, bcs, 0, stream)))
+    return st;
   if (order == 3) {
     if ((st = run_stage(grid, scheme, ext, (const void* const*)out, cu0, w,
-                        SWC_OUT_CONVEX, 0.75, 0.25, dt, stream)))
+                        SWC_OUT_CONVEX, 0.75, 0.25, dt, from, stream)))
       return st;
-    if ((st = swc_halo_fill(grid, dtype, nf, w, bcs, 0, stream))) return st;
+    if (!mapped && (st = swc_halo_fill(grid, dtype, nf, w, bcs, 0, stream)))
+      return st;
     st = run_stage(grid, scheme, ext, (const void* const*)w, cu0, out,
-                   SWC_OUT_CONVEX, 1.0 / 3.0, 2.0 / 3.0, dt, stream);
+                   SWC_OUT_CONVEX, 1.0 / 3.0, 2.0 / 3.0, dt, from, stream);
   } else {
     st = run_stage(grid, scheme, ext, (const void* const*)w, cu0, out,
-                   SWC_OUT_AVERAGE, 0.5, 0.0, dt, stream);
+                   SWC_OUT_AVERAGE, 0.5, 0.0, dt, from, stream);
   }
   if (st) return st;
   return swc_halo_fill(grid, dtype, nf, out, bcs, 0, stream);

@@ -2,7 +2,7 @@
 // per-element routine shared by the single-grid and the batched passes.
 #pragma once
 
-#include "swc_physics.cuh"
+#include "swc_stage.cuh"
 #include "swirlc_b200.h"
 
 namespace swc {
@@ -257,11 +257,10 @@ struct ShellArgs {
   ShellField fld[SWC_MAX_FIELDS];
   int nx, ny, nz, h;
   long long sx, sz;
-  // Per dim: kShellWrap where every field is periodic, kShellClamp where every
-  // field has Neumann sides of slope 0, else kShellMixed.
+  // Per dim: kHaloWrapped where every field is periodic, kHaloClamped where
+  // every field has Neumann sides of slope 0, else kHaloStored.
   int dims[3];
 };
-enum { kShellMixed, kShellWrap, kShellClamp };
 
 // Offset of the interior cell that every field copies at the padded cell
 // (cx, cy, cz) (its own for an interior cell). False where the cell lies in
@@ -271,11 +270,9 @@ __device__ __forceinline__ bool shell_source(const ShellArgs& a, int cx, int cy,
                                              int cz, long long& os) {
   const int h = a.h;
   bool same = true;
-  auto src = [&](int c, int n, int kind) {
-    if (c >= h && c < n + h) return c;
-    if (kind == kShellMixed) same = false;
-    if (kind == kShellWrap) return c < h ? c + n : c - n;
-    return c < h ? h : n + h - 1;
+  auto src = [&](int c, int n, int from) {
+    if (from == kHaloStored && (c < h || c >= n + h)) same = false;
+    return halo_source(c, n, h, from);
   };
   const int x = src(cx, a.nx, a.dims[0]), y = src(cy, a.ny, a.dims[1]);
   os = src(cz, a.nz, a.dims[2]) * a.sz + x * a.sx + y;
@@ -337,6 +334,17 @@ __device__ __forceinline__ T halo_shell_value(const ShellArgs& a,
     for (int l = 0; l < nl[d]; ++l) val = ns[d] == 0 ? val - inc : val + inc;
   }
   return val;
+}
+
+// Zeros in element t of the halo shell of nf fields.
+template <typename T>
+__device__ __forceinline__ void halo_clear_elem(const ShellArgs& a, int t) {
+  int cx, cy, cz;
+  shell_cell(a.h, a.nx, a.ny, a.nz, t, cx, cy, cz);
+  const long long o = cz * a.sz + cx * a.sx + cy;
+#pragma unroll
+  for (int f = 0; f < SWC_MAX_FIELDS; ++f)
+    if (f < a.nf) static_cast<T*>(a.fld[f].f)[o] = T(0);
 }
 
 template <typename T>
