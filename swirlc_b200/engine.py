@@ -581,9 +581,10 @@ class Solver:
 class Stepper:
   """In-place time loop over a state with a device clock (no host syncs).
 
-  Each step: [clock begin] -> fill(u) -> stage EULER u->w1 -> fill(w1) ->
-  stage CONVEX (u, w1)->w2 -> fill(w2) -> stage CONVEX (u, w2)->u with the
-  fused CFL reduction -> [clock end]. With `cfl` > 0 the step size is
+  Each step: fill(u), which advances the clock -> stage EULER u->w1 ->
+  fill(w1) -> stage CONVEX (u, w1)->w2 -> fill(w2) -> stage CONVEX (u, w2)->u
+  with the fused CFL reduction; the fills of w1 and w2 fall away where the
+  stages read their halos from the interior. With `cfl` > 0 the step size is
   cfl * min(delta/(|u|+c)) computed on the device.
   """
 

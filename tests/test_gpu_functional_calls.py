@@ -1,7 +1,7 @@
 """GPU: the functional calls (swc_halo_copy, swc_rhs, swc_rk_step_out) give the
 bits of their composition from copies, halo fills and stages, for every kind of
 boundary condition, at the edges of the copy's blocks (32 cells along y, 8
-along x), and leave the caller's fields as they are."""
+rows of two cells along x), and leave the caller's fields as they are."""
 
 import ctypes
 
