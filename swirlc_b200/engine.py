@@ -492,11 +492,13 @@ class Solver:
   # allocation. With replicas the halos come from other ranks between the
   # stages, so the steps are composed here.
   def _ext_of(self, helper):
-    """The stage's SwcStageExt, or None for the plain stage."""
+    """The stage's SwcStageExt, or None for the plain stage. It holds the
+    reference states it points at: a list of slices is stacked into a tensor
+    nobody else keeps, whose memory the next allocation would be given."""
     if helper:
       e = nat.SwcStageExt.from_buffer_copy(self.ext)
-      e.p_ref = self._helper_field(helper, 'p_ref').data_ptr()
-      e.rho_ref = self._helper_field(helper, 'rho_ref').data_ptr()
+      e.held = tuple(self._helper_field(helper, n) for n in ('p_ref', 'rho_ref'))
+      e.p_ref, e.rho_ref = (t.data_ptr() for t in e.held)
       return e
     return self.ext if self.use_ext else None
 
