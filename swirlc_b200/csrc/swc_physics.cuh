@@ -291,23 +291,25 @@ struct CellStencil<3> {
 // with eps = 1e-6, the smoothness indicators
 // beta_r = 13/12 a_r^2 + 1/4 b_r^2 and the candidate polynomials q_r of the
 // reference prototype's `weno5`; the value is sum alpha_r q_r / sum alpha_r.
-// It is evaluated as the central candidate plus a correction. With the first
-// differences e_k = v[k+1] - v[k] of the stencil, a_r is the second
-// difference of candidate r's three cells (e_hi - e_lo), and q_0 - q_1,
-// q_2 - q_1 are multiples of the third differences t_up = a_0 - a_1 and
-// t_lo = a_1 - a_2 (weights w_r = 1/beta_r^2 up to a common factor):
-//   right (c+1/2): v0 + dm1/6 + d0/3 - (w0 t_up + 2/3 w2 t_lo) /
-//                                      (6 w0 + 12 w1 + 2 w2)
-//   left  (c-1/2): v0 - dm1/3 - d0/6 + (2/3 w0 t_up + w2 t_lo) /
-//                                      (2 w0 + 12 w1 + 6 w2)
-// (d = (0.3, 0.6, 0.1) and mirrored, the common factor 1/20 divided out).
-// That is 41 products and sums for both faces of a cell, against 54 with the
-// three candidates spelled out, and a uniform field comes out unrounded. The
-// differences are shared: by the two faces of a cell and, in the face form,
-// by the two cells.
+// It is evaluated as v0 plus the weighted mean of the candidates' offsets
+// q_r - v0, each written in the first differences e_k = v[k+1] - v[k] of its
+// own three cells (dm2, dm1, d0, d1 around the cell; weights
+// w_r = 1/beta_r^2 up to a common factor; d = (0.3, 0.6, 0.1) and mirrored):
+//   right (c+1/2): v0 + (w0 (4 d0 - d1) + 2 w1 (dm1 + 2 d0)
+//                        + w2 (5 dm1 - 2 dm2) / 3) / (6 w0 + 12 w1 + 2 w2)
+//   left  (c-1/2): v0 - (w2 (4 dm1 - dm2) + 2 w1 (d0 + 2 dm1)
+//                        + w0 (5 d0 - 2 d1) / 3) / (2 w0 + 12 w1 + 6 w2)
+// A candidate whose cells hold a jump J enters with J times its weight of
+// about J^-4 only, so a face value is accurate to a few units in the last
+// place of what lies on its own side. (The shorter form of a central candidate
+// and a correction in third differences has two terms of size J that cancel:
+// 2e-4 of a low side of 0.01 beside 1000 in single precision.) A uniform
+// field comes out unrounded. The differences are shared: by the two faces of
+// a cell and, in the face form, by the two cells.
 // B_r = 4 (beta_r + eps) = 13/3 a_r^2 + (b_r^2 + 4 eps), so eps folds into an
-// FMA; b_r = e_hi - 3 e_lo (r = 0), e_lo + e_hi (r = 1), e_lo - 3 e_hi
-// (r = 2) up to sign.
+// FMA; a_r is the second difference e_hi - e_lo of candidate r's three cells,
+// b_r = e_hi - 3 e_lo (r = 0), e_lo + e_hi (r = 1), e_lo - 3 e_hi (r = 2) up
+// to sign.
 // Weights. Single precision: w_r = 1/B_r^2 by the hardware reciprocal.
 // Double precision, where a reciprocal is a long sequence: w_0 = (B_1 B_2)^2
 // and so on, no reciprocal, formed from differences scaled by 2^-116 so that
@@ -371,36 +373,42 @@ __device__ __forceinline__ Weno5W<O> weno5_weights(
             O::rcp(O::mul(b2, b2))};
   }
 }
-template <class O>
-__device__ __forceinline__ typename O::V weno5_right_v(
-    const Weno5W<O>& w, typename O::V v0, typename O::V dm1,
-    typename O::V d0, typename O::V t_up, typename O::V t_lo) {
+// The face value on one side of a cell: wn, wf are the weights of the
+// candidates that reach farthest towards the face and away from it; dn, dn1
+// (df, df1) the first and second of the differences on those two sides.
+// RIGHT: w0, w2, d0, d1, dm1, dm2; left: w2, w0, dm1, dm2, d0, d1. The mean
+// offset is formed with both signs turned on the right (FMAs of two lanes
+// have no negated operand).
+template <class O, bool RIGHT>
+__device__ __forceinline__ typename O::V weno5_side_v(
+    typename O::V wn, typename O::V w1, typename O::V wf, typename O::V v0,
+    typename O::V dn, typename O::V dn1, typename O::V df,
+    typename O::V df1) {
   using S = typename O::S;
   using V = typename O::V;
-  const V q = O::fma(O::splat(S(1.0 / 3.0)), d0,
-                     O::fma(O::splat(S(1.0 / 6.0)), dm1, v0));
-  const V num = O::fma(O::splat(S(2.0 / 3.0)), O::mul(w.w2, t_lo),
-                       O::mul(w.w0, t_up));
-  // The denominator with the sign of the correction.
-  const V den = O::fma(O::splat(S(-6)), w.w0,
-                       O::fma(O::splat(S(-2)), w.w2,
-                              O::mul(O::splat(S(-12)), w.w1)));
-  return O::fma(num, O::rcpn(den), q);
+  const V on = O::fma(O::splat(S(-4)), dn, dn1);
+  const V o1 = O::fma(O::splat(S(2)), dn, df);
+  const V of = O::fma(O::splat(S(-2.5)), df, df1);
+  const V m1 = O::mul(O::splat(S(-2)), w1);
+  const V mf = O::mul(O::splat(S(2.0 / 3.0)), wf);
+  const V num = O::fma(mf, of, O::fma(m1, o1, O::mul(wn, on)));
+  const S s = RIGHT ? S(-1) : S(1);
+  const V den = O::fma(O::splat(s * S(2)), wf,
+                       O::fma(O::splat(s * S(12)), w1,
+                              O::mul(O::splat(s * S(6)), wn)));
+  return O::fma(num, O::rcpn(den), v0);
+}
+template <class O>
+__device__ __forceinline__ typename O::V weno5_right_v(
+    const Weno5W<O>& w, typename O::V v0, typename O::V dm2,
+    typename O::V dm1, typename O::V d0, typename O::V d1) {
+  return weno5_side_v<O, true>(w.w0, w.w1, w.w2, v0, d0, d1, dm1, dm2);
 }
 template <class O>
 __device__ __forceinline__ typename O::V weno5_left_v(
-    const Weno5W<O>& w, typename O::V v0, typename O::V dm1,
-    typename O::V d0, typename O::V t_up, typename O::V t_lo) {
-  using S = typename O::S;
-  using V = typename O::V;
-  const V q = O::fma(O::splat(S(-1.0 / 6.0)), d0,
-                     O::fma(O::splat(S(-1.0 / 3.0)), dm1, v0));
-  const V num = O::fma(O::splat(S(2.0 / 3.0)), O::mul(w.w0, t_up),
-                       O::mul(w.w2, t_lo));
-  const V den = O::fma(O::splat(S(2)), w.w0,
-                       O::fma(O::splat(S(6)), w.w2,
-                              O::mul(O::splat(S(12)), w.w1)));
-  return O::fma(num, O::rcpn(den), q);
+    const Weno5W<O>& w, typename O::V v0, typename O::V dm2,
+    typename O::V dm1, typename O::V d0, typename O::V d1) {
+  return weno5_side_v<O, false>(w.w2, w.w1, w.w0, v0, dm1, dm2, d0, d1);
 }
 
 // WENO3 (k = 2) on v[c-1..c+1], d0 = v[c+1]-v[c], dm = v[c]-v[c-1]: weights
@@ -473,9 +481,9 @@ __device__ __forceinline__ void recon_face(const typename O::V* s, int limiter,
   using S = typename O::S;
   using V = typename O::V;
   if constexpr (SCHEME == 0) {
-    // Cells i-1 (s[0..4]) and i (s[1..5]) share the differences e1..e3, the
-    // second differences f1, f2 and the third difference t1.
-    V e[5], d[5], t[3];
+    // Cells i-1 (s[0..4]) and i (s[1..5]) share the differences e1..e3 and the
+    // second differences f1, f2.
+    V e[5], d[5];
 #pragma unroll
     for (int k = 0; k < 5; ++k) {
       e[k] = O::sub(s[k + 1], s[k]);
@@ -484,14 +492,12 @@ __device__ __forceinline__ void recon_face(const typename O::V* s, int limiter,
     Weno5Tri<O> f[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) f[k] = weno5_tri<O>(e[k], e[k + 1]);
-#pragma unroll
-    for (int k = 0; k < 3; ++k) t[k] = O::sub(f[k + 1].a, f[k].a);
     neg = weno5_right_v<O>(
         weno5_weights<O>(f[0], f[1], f[2], d[0], d[1], d[2], d[3]), s[2],
-        e[1], e[2], t[1], t[0]);
+        e[0], e[1], e[2], e[3]);
     pos = weno5_left_v<O>(
         weno5_weights<O>(f[1], f[2], f[3], d[1], d[2], d[3], d[4]), s[3],
-        e[2], e[3], t[2], t[1]);
+        e[1], e[2], e[3], e[4]);
   } else if constexpr (SCHEME == 1) {
     V w0, w1;
     const V d0 = O::sub(s[1], s[0]), d1 = O::sub(s[2], s[1]),
@@ -528,11 +534,10 @@ __device__ __forceinline__ void recon_cell(const typename O::V* s, int limiter,
     Weno5Tri<O> f[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) f[k] = weno5_tri<O>(e[k], e[k + 1]);
-    const V t_lo = O::sub(f[1].a, f[0].a), t_up = O::sub(f[2].a, f[1].a);
     const Weno5W<O> w =
         weno5_weights<O>(f[0], f[1], f[2], d[0], d[1], d[2], d[3]);
-    right = weno5_right_v<O>(w, s[2], e[1], e[2], t_up, t_lo);
-    left = weno5_left_v<O>(w, s[2], e[1], e[2], t_up, t_lo);
+    right = weno5_right_v<O>(w, s[2], e[0], e[1], e[2], e[3]);
+    left = weno5_left_v<O>(w, s[2], e[0], e[1], e[2], e[3]);
   } else if constexpr (SCHEME == 1) {
     V w0, w1;
     const V dm = O::sub(s[1], s[0]), d0 = O::sub(s[2], s[1]);
