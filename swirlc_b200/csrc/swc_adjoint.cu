@@ -23,6 +23,7 @@
 #include <string.h>
 
 #include "swc_launch.h"
+#include "swc_recon_vjp.cuh"
 #include "swirlc_b200.h"
 
 namespace swc {
@@ -31,76 +32,6 @@ namespace {
 // ---------------------------------------------------------------------------
 // Reverse of the pieces of one face flux.
 // ---------------------------------------------------------------------------
-
-// Reverse of recon_cell<0, O> (swc_physics.cuh) on one or two variables
-// (the lanes of O): both WENO5 face values of the cell v[2] from
-// v[0..4] = v[c-2 .. c+2], which share the smoothness indicators.
-// vb[k] += d right/dv[k] * rb + d left/dv[k] * lb. The forward is that of
-// weno5_right_v / weno5_left_v: first differences e, second differences f,
-// third differences t_lo, t_up, B_r = 13/3 a_r^2 + b_r^2 + 4 eps,
-// w_r = 1/B_r^2 and each face value a central candidate plus num / den. With
-// c = num / den and g = cotangent / den of a face (den with the sign of the
-// correction, as there), d num = g and d den = -g c; the differences'
-// cotangents move onto the cells last. 92 products and sums and 5
-// reciprocals per cell, against 150 with the three candidates of each face
-// spelled out.
-template <class O>
-__device__ __forceinline__ void weno5_cell_vjp_v(const typename O::V* v,
-                                                 typename O::V rb,
-                                                 typename O::V lb,
-                                                 typename O::V* vb) {
-  using S = typename O::S;
-  using V = typename O::V;
-  auto k = [](double c) -> V { return O::splat(S(c)); };
-  const V e0 = O::sub(v[1], v[0]), e1 = O::sub(v[2], v[1]);
-  const V e2 = O::sub(v[3], v[2]), e3 = O::sub(v[4], v[3]);
-  // a_2, a_1, a_0 of the candidates r = 2, 1, 0.
-  const V f0 = O::sub(e1, e0), f1 = O::sub(e2, e1), f2 = O::sub(e3, e2);
-  const V t_lo = O::sub(f1, f0), t_up = O::sub(f2, f1);
-  const V c0 = O::mul(k(13.0 / 3.0), f0), c1 = O::mul(k(13.0 / 3.0), f1);
-  const V c2 = O::mul(k(13.0 / 3.0), f2);
-  const V b0 = O::fma(k(-3), e2, e3), b1 = O::add(e2, e1);
-  const V b2 = O::fma(k(-3), e1, e0);
-  const V eps = k(4e-6);
-  const V i0 = O::rcp(O::fma(c2, f2, O::fma(b0, b0, eps)));
-  const V i1 = O::rcp(O::fma(c1, f1, O::fma(b1, b1, eps)));
-  const V i2 = O::rcp(O::fma(c0, f0, O::fma(b2, b2, eps)));
-  const V w0 = O::mul(i0, i0), w1 = O::mul(i1, i1), w2 = O::mul(i2, i2);
-  const V p0 = O::mul(w0, t_up), p2 = O::mul(w2, t_lo), m1 = O::mul(k(12), w1);
-  const V dr = O::rcp(O::fma(k(-6), w0, O::fma(k(-2), w2, O::mul(k(-1), m1))));
-  const V dl = O::rcp(O::fma(k(2), w0, O::fma(k(6), w2, m1)));
-  const V cr = O::mul(O::fma(k(2.0 / 3.0), p2, p0), dr);
-  const V cl = O::mul(O::fma(k(2.0 / 3.0), p0, p2), dl);
-  const V gr = O::mul(rb, dr), gl = O::mul(lb, dl);
-  const V hr = O::mul(gr, cr), hl = O::mul(gl, cl);
-  const V s0 = O::fma(k(2.0 / 3.0), gl, gr), s2 = O::fma(k(2.0 / 3.0), gr, gl);
-  // Cotangents of the weights, then x_r = 2 dB_r = -4 w_r / B_r dw_r.
-  const V y0 = O::fma(t_up, s0, O::fma(k(6), hr, O::mul(k(-2), hl)));
-  const V y1 = O::mul(k(12), O::sub(hr, hl));
-  const V y2 = O::fma(t_lo, s2, O::fma(k(2), hr, O::mul(k(-6), hl)));
-  const V x0 = O::mul(O::mul(k(-4), O::mul(w0, i0)), y0);
-  const V x1 = O::mul(O::mul(k(-4), O::mul(w1, i1)), y1);
-  const V x2 = O::mul(O::mul(k(-4), O::mul(w2, i2)), y2);
-  // Cotangents of t_up, t_lo, of the second and of the first differences.
-  const V tu = O::mul(w0, s0), tl = O::mul(w2, s2);
-  const V g0 = O::sub(O::mul(c0, x2), tl);
-  const V g1 = O::fma(c1, x1, O::sub(tl, tu));
-  const V g2 = O::fma(c2, x0, tu);
-  const V z0 = O::mul(b0, x0), z1 = O::mul(b1, x1), z2 = O::mul(b2, x2);
-  const V d0 = O::sub(z2, g0);
-  const V d1 = O::add(O::fma(k(-3), z2, z1),
-                      O::add(O::sub(g0, g1), O::fma(k(1.0 / 6.0), rb,
-                                                    O::mul(k(-1.0 / 3.0), lb))));
-  const V d2 = O::add(O::fma(k(-3), z0, z1),
-                      O::add(O::sub(g1, g2), O::fma(k(1.0 / 3.0), rb,
-                                                    O::mul(k(-1.0 / 6.0), lb))));
-  const V d3 = O::add(z0, g2);
-  vb[0] = O::sub(vb[0], d0);
-  vb[1] = O::add(vb[1], O::sub(d0, d1));
-  vb[2] = O::add(vb[2], O::add(O::add(rb, lb), O::sub(d1, d2)));
-  vb[3] = O::add(vb[3], O::sub(d2, d3));
-  vb[4] = O::add(vb[4], d3);
-}
 
 // Primitive cotangents of one face state, rotated frame (u[0] normal).
 template <typename T>
