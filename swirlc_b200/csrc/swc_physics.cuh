@@ -8,6 +8,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 namespace swc {
 
 // physics/constant.py:17-41. Python doubles rounded once to T, as TF does
@@ -71,6 +73,46 @@ __device__ __forceinline__ double rcp_normal(double a) {
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(a));
   const double r = __fma_rn(-a, x, 1.0);
   return __fma_rn(__fma_rn(r, r, r), x, x);
+}
+// w_r = 1/b_r^2 up to a common factor, for positive b_r, without reciprocals:
+// w_0 = (b_1 b_2 s)^2 and so on. The power of two s brings the largest product
+// to [1, 2), so that no weight that counts leaves the normal range, however
+// large or small the b_r. b_r above 2^511, whose squares overflow, count as
+// 2^511. Two steps of KH 112^3: 1238 us; with one reciprocal per b_r 1281;
+// with a fixed scale, whose products leave the normal range for fields below
+// 1e-8 and above 1e62, 1193.
+__device__ __forceinline__ double limit_511(double b) {
+  const int hi = __double2hiint(b);
+  return __hiloint2double(hi < 0x5fe00000 ? hi : 0x5fe00000, __double2loint(b));
+}
+// 2^-e for a product p = 2^e f, 1 <= f < 2, given by its upper word.
+__device__ __forceinline__ double unit_scale(int hi) {
+  return __hiloint2double(0x7fe00000 - (hi & 0x7ff00000), 0);
+}
+__device__ __forceinline__ void inv_squares(double b0, double b1, double b2,
+                                            double& w0, double& w1,
+                                            double& w2) {
+  b0 = limit_511(b0);
+  b1 = limit_511(b1);
+  b2 = limit_511(b2);
+  const double p0 = __dmul_rn(b1, b2), p1 = __dmul_rn(b0, b2);
+  const double p2 = __dmul_rn(b0, b1);
+  const double s = unit_scale(max(max(__double2hiint(p0), __double2hiint(p1)),
+                                  __double2hiint(p2)));
+  const double q0 = __dmul_rn(p0, s), q1 = __dmul_rn(p1, s);
+  const double q2 = __dmul_rn(p2, s);
+  w0 = __dmul_rn(q0, q0);
+  w1 = __dmul_rn(q1, q1);
+  w2 = __dmul_rn(q2, q2);
+}
+__device__ __forceinline__ void inv_squares(double b0, double b1, double& w0,
+                                            double& w1) {
+  b0 = limit_511(b0);
+  b1 = limit_511(b1);
+  const double s = unit_scale(max(__double2hiint(b0), __double2hiint(b1)));
+  const double q0 = __dmul_rn(b1, s), q1 = __dmul_rn(b0, s);
+  w0 = __dmul_rn(q0, q0);
+  w1 = __dmul_rn(q1, q1);
 }
 
 // ---------------------------------------------------------------------------
@@ -310,48 +352,31 @@ struct CellStencil<3> {
 // FMA; a_r is the second difference e_hi - e_lo of candidate r's three cells,
 // b_r = e_hi - 3 e_lo (r = 0), e_lo + e_hi (r = 1), e_lo - 3 e_hi (r = 2) up
 // to sign.
-// Weights. Single precision: w_r = 1/B_r^2 by the hardware reciprocal.
-// Double precision, where a reciprocal is a long sequence: w_0 = (B_1 B_2)^2
-// and so on, no reciprocal, formed from differences scaled by 2^-116 so that
-// the products stay normal for jumps up to 1e72.
+// w_r = 1/B_r^2: by the hardware reciprocal in single precision, up to a common
+// factor in double (inv_squares). Jumps reach up to 2e9 and 1e76.
 template <class O>
-struct Weno5Tri {  // second difference a of three cells and 13/3 a (scaled)
+struct Weno5Tri {  // second difference a of three cells and 13/3 a
   typename O::V a, ca;
-};
-template <class O>
-struct Weno5Scale {
-  static constexpr bool kWide = sizeof(typename O::S) == 8;
-  // 2^-116 and its square.
-  static constexpr double kS = kWide ? 0x1p-116 : 1.0;
-  static constexpr double kS2 = kWide ? 0x1p-232 : 1.0;
 };
 template <class O>
 __device__ __forceinline__ Weno5Tri<O> weno5_tri(typename O::V e_lo,
                                                  typename O::V e_hi) {
   using S = typename O::S;
   const typename O::V a = O::sub(e_hi, e_lo);
-  return {a, O::mul(O::splat(S(13.0 / 3.0 * Weno5Scale<O>::kS2)), a)};
+  return {a, O::mul(O::splat(S(13.0 / 3.0)), a)};
 }
-template <class O>
-__device__ __forceinline__ typename O::V weno5_scaled(typename O::V e) {
-  if constexpr (Weno5Scale<O>::kWide)
-    return O::mul(O::splat(typename O::S(Weno5Scale<O>::kS)), e);
-  else
-    return e;
-}
-// 4 (beta + eps) = 13/3 a^2 + (b^2 + 4 eps), scaled.
+// 4 (beta + eps) = 13/3 a^2 + (b^2 + 4 eps).
 template <class O>
 __device__ __forceinline__ typename O::V weno5_b4(const Weno5Tri<O>& t,
                                                   typename O::V b) {
   using S = typename O::S;
-  return O::fma(t.ca, t.a,
-                O::fma(b, b, O::splat(S(4e-6 * Weno5Scale<O>::kS2))));
+  return O::fma(t.ca, t.a, O::fma(b, b, O::splat(S(4e-6))));
 }
 template <class O>
 struct Weno5W {
   typename O::V w0, w1, w2;
 };
-// Cell with the scaled differences dm2 = v[c-1]-v[c-2], dm1 = v[c]-v[c-1],
+// Cell with the differences dm2 = v[c-1]-v[c-2], dm1 = v[c]-v[c-1],
 // d0 = v[c+1]-v[c], d1 = v[c+2]-v[c+1] and the second differences
 // t2 = (dm2, dm1), t1 = (dm1, d0), t0 = (d0, d1).
 template <class O>
@@ -365,13 +390,17 @@ __device__ __forceinline__ Weno5W<O> weno5_weights(
   const V b0 = weno5_b4<O>(t0, O::fma(m3, d0, d1));
   const V b1 = weno5_b4<O>(t1, O::add(d0, dm1));
   const V b2 = weno5_b4<O>(t2, O::fma(m3, dm1, dm2));
-  if constexpr (Weno5Scale<O>::kWide) {
-    const V p0 = O::mul(b1, b2), p1 = O::mul(b0, b2), p2 = O::mul(b0, b1);
-    return {O::mul(p0, p0), O::mul(p1, p1), O::mul(p2, p2)};
+  Weno5W<O> w;
+  if constexpr (std::is_same<V, double>::value) {
+    inv_squares(b0, b1, b2, w.w0, w.w1, w.w2);
+  } else if constexpr (std::is_same<V, double2>::value) {
+    inv_squares(b0.x, b1.x, b2.x, w.w0.x, w.w1.x, w.w2.x);
+    inv_squares(b0.y, b1.y, b2.y, w.w0.y, w.w1.y, w.w2.y);
   } else {
-    return {O::rcp(O::mul(b0, b0)), O::rcp(O::mul(b1, b1)),
-            O::rcp(O::mul(b2, b2))};
+    w = {O::rcp(O::mul(b0, b0)), O::rcp(O::mul(b1, b1)),
+         O::rcp(O::mul(b2, b2))};
   }
+  return w;
 }
 // The face value on one side of a cell: wn, wf are the weights of the
 // candidates that reach farthest towards the face and away from it; dn, dn1
@@ -425,9 +454,11 @@ __device__ __forceinline__ void weno3_weights(typename O::V d0,
   using V = typename O::V;
   const V eps = O::splat(S(1e-6));
   const V b0 = O::fma(d0, d0, eps), b1 = O::fma(dm, dm, eps);
-  if constexpr (sizeof(S) == 8) {
-    w0 = O::mul(b1, b1);
-    w1 = O::mul(b0, b0);
+  if constexpr (std::is_same<V, double>::value) {
+    inv_squares(b0, b1, w0, w1);
+  } else if constexpr (std::is_same<V, double2>::value) {
+    inv_squares(b0.x, b1.x, w0.x, w1.x);
+    inv_squares(b0.y, b1.y, w0.y, w1.y);
   } else {
     w0 = O::rcp(O::mul(b0, b0));
     w1 = O::rcp(O::mul(b1, b1));
@@ -483,20 +514,17 @@ __device__ __forceinline__ void recon_face(const typename O::V* s, int limiter,
   if constexpr (SCHEME == 0) {
     // Cells i-1 (s[0..4]) and i (s[1..5]) share the differences e1..e3 and the
     // second differences f1, f2.
-    V e[5], d[5];
+    V e[5];
 #pragma unroll
-    for (int k = 0; k < 5; ++k) {
-      e[k] = O::sub(s[k + 1], s[k]);
-      d[k] = weno5_scaled<O>(e[k]);
-    }
+    for (int k = 0; k < 5; ++k) e[k] = O::sub(s[k + 1], s[k]);
     Weno5Tri<O> f[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) f[k] = weno5_tri<O>(e[k], e[k + 1]);
     neg = weno5_right_v<O>(
-        weno5_weights<O>(f[0], f[1], f[2], d[0], d[1], d[2], d[3]), s[2],
+        weno5_weights<O>(f[0], f[1], f[2], e[0], e[1], e[2], e[3]), s[2],
         e[0], e[1], e[2], e[3]);
     pos = weno5_left_v<O>(
-        weno5_weights<O>(f[1], f[2], f[3], d[1], d[2], d[3], d[4]), s[3],
+        weno5_weights<O>(f[1], f[2], f[3], e[1], e[2], e[3], e[4]), s[3],
         e[1], e[2], e[3], e[4]);
   } else if constexpr (SCHEME == 1) {
     V w0, w1;
@@ -525,17 +553,14 @@ __device__ __forceinline__ void recon_cell(const typename O::V* s, int limiter,
   using S = typename O::S;
   using V = typename O::V;
   if constexpr (SCHEME == 0) {
-    V e[4], d[4];
+    V e[4];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      e[k] = O::sub(s[k + 1], s[k]);
-      d[k] = weno5_scaled<O>(e[k]);
-    }
+    for (int k = 0; k < 4; ++k) e[k] = O::sub(s[k + 1], s[k]);
     Weno5Tri<O> f[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) f[k] = weno5_tri<O>(e[k], e[k + 1]);
     const Weno5W<O> w =
-        weno5_weights<O>(f[0], f[1], f[2], d[0], d[1], d[2], d[3]);
+        weno5_weights<O>(f[0], f[1], f[2], e[0], e[1], e[2], e[3]);
     right = weno5_right_v<O>(w, s[2], e[0], e[1], e[2], e[3]);
     left = weno5_left_v<O>(w, s[2], e[0], e[1], e[2], e[3]);
   } else if constexpr (SCHEME == 1) {
