@@ -198,10 +198,14 @@ int swc_rk_stage_ext(const SwcGrid* grid, const SwcScheme* scheme,
                      double c0, double c1, const double* dt,
                      double* dtmin_out, void* stream);
 
-/* One time step in place on `u` (5 fields): [clock begin] -> halo fill ->
- * fused stages -> [clock end]. order 3: SSP-RK3 (rk3.py:87-120); order 2:
- * RK2 (rk2.py:69-86). `work` holds 10 field buffers (two states of the
- * shape of u) used as scratch. `clock_dev` is a device SwcClock: the step
+/* One time step in place on `u` (5 fields): halo fill of u, which also moves
+ * the clock (dt chosen, then t and step), and the fused stages; the stages
+ * between read halos from the interior cells they copy, or after fills of
+ * their own where a condition needs one. order 3: SSP-RK3 (rk3.py:87-120);
+ * order 2: RK2 (rk2.py:69-86). `work` holds 10 field buffers (two states of
+ * the shape of u) used as scratch; their halos may stay unwritten. A call
+ * that is refused (SWC_ERR_ARG, SWC_ERR_UNSUPPORTED) launches nothing and
+ * leaves the clock as it is. `clock_dev` is a device SwcClock: the step
  * uses clock->dt; with clock->cfl > 0 the step starts with
  * dt = min(cfl*dtmin, t_end-t) and its last stage min-reduces the CFL limit
  * of the new state into clock->dtmin for the next step (so before the first

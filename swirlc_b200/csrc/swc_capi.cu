@@ -858,19 +858,21 @@ static int stage_args(const SwcGrid* grid, const SwcScheme* sc, int nf,
   return SWC_OK;
 }
 
-static int plain_stage(const SwcGrid* grid, const SwcScheme* sc,
-                       const void* const* uk, const void* const* u0,
-                       void* const* uout, int32_t mode, double c0, double c1,
-                       const double* dt, double* dtmin_out,
-                       const HaloFrom& from, void* stream) {
-  swc::NvtxRange nvtx_range_("swc_rk_stage");
+// Checks and arguments of the plain stage.
+static int plain_args(const SwcGrid* grid, const SwcScheme* sc,
+                      const void* const* uk, const void* const* u0,
+                      void* const* uout, int32_t mode, double c0, double c1,
+                      const double* dt, double* dtmin_out,
+                      const HaloFrom& from, StageArgs& a) {
   if (sc && sc->nscalars != 0)
     return fail(SWC_ERR_UNSUPPORTED,
                 "transported scalars go through swc_rk_stage_ext");
-  StageArgs a;
-  int st = stage_args(grid, sc, 5, uk, u0, uout, mode, c0, c1, dt, dtmin_out,
-                      from, a);
-  if (st) return st;
+  return stage_args(grid, sc, 5, uk, u0, uout, mode, c0, c1, dt, dtmin_out,
+                    from, a);
+}
+
+static int plain_launch(const SwcScheme* sc, const StageArgs& a, void* stream) {
+  swc::NvtxRange nvtx_range_("swc_rk_stage");
   const int visc = sc->diffusion ? 1 : 0;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   int rc;
@@ -891,6 +893,17 @@ static int plain_stage(const SwcGrid* grid, const SwcScheme* sc,
   }
   if (rc) return fail(rc, "stage launch failed: %s", cudaGetErrorString(cudaGetLastError()));
   return SWC_OK;
+}
+
+static int plain_stage(const SwcGrid* grid, const SwcScheme* sc,
+                       const void* const* uk, const void* const* u0,
+                       void* const* uout, int32_t mode, double c0, double c1,
+                       const double* dt, double* dtmin_out,
+                       const HaloFrom& from, void* stream) {
+  StageArgs a;
+  const int st = plain_args(grid, sc, uk, u0, uout, mode, c0, c1, dt,
+                            dtmin_out, from, a);
+  return st ? st : plain_launch(sc, a, stream);
 }
 
 int swc_rk_stage(const SwcGrid* grid, const SwcScheme* sc,
@@ -1297,31 +1310,41 @@ int swc_rk_step(const SwcGrid* grid, const SwcScheme* scheme,
   }
   const double* dt = &clock_dev->dt;
   double* dtmin = &clock_dev->dtmin;
-  if ((st = halo_fill(grid, scheme->dtype, 5, u, bcs, 0, clock_dev, stream)))
+  const void* const* cu = (const void* const*)u;
+  // Everything is checked before the first launch: the step's first fill moves
+  // the clock, which a refused step leaves as it is.
+  bool any_prim = false;
+  if ((st = check_halo(grid, scheme->dtype, 5, cu, bcs, 0, &any_prim)))
     return st;
   // The work states' halos are read from the interior where they can be.
-  bool any_prim = false;
-  for (int v = 0; v < 5; ++v) any_prim |= bcs[v].via_primitive != 0;
   HaloFrom from;
-  const bool fill = !halo_from_interior(grid, 5, (const void* const*)u, bcs,
-                                        any_prim, &from);
-  const void* const* cu = (const void* const*)u;
-  if ((st = plain_stage(grid, scheme, cu, nullptr, w1, SWC_OUT_EULER, 0.0, 0.0,
-                        dt, nullptr, kAllStored, stream)))
+  const bool fill = !halo_from_interior(grid, 5, cu, bcs, any_prim, &from);
+  StageArgs a[3];
+  if ((st = plain_args(grid, scheme, cu, nullptr, w1, SWC_OUT_EULER, 0.0, 0.0,
+                       dt, nullptr, kAllStored, a[0])))
     return st;
-  if (fill && (st = swc_halo_fill(grid, scheme->dtype, 5, w1, bcs, 0, stream)))
+  if (order == 2) {
+    st = plain_args(grid, scheme, (const void* const*)w1, cu, u,
+                    SWC_OUT_AVERAGE, 0.5, 0.0, dt, dtmin, from, a[1]);
+  } else {
+    st = plain_args(grid, scheme, (const void* const*)w1, cu, w2,
+                    SWC_OUT_CONVEX, 0.75, 0.25, dt, nullptr, from, a[1]);
+    if (!st)
+      st = plain_args(grid, scheme, (const void* const*)w2, cu, u,
+                      SWC_OUT_CONVEX, 1.0 / 3.0, 2.0 / 3.0, dt, dtmin, from,
+                      a[2]);
+  }
+  if (st) return st;
+  if ((st = halo_fill(grid, scheme->dtype, 5, u, bcs, 0, clock_dev, stream)))
     return st;
-  if (order == 2)
-    return plain_stage(grid, scheme, (const void* const*)w1, cu, u,
-                       SWC_OUT_AVERAGE, 0.5, 0.0, dt, dtmin, from, stream);
-  if ((st = plain_stage(grid, scheme, (const void* const*)w1, cu, w2,
-                        SWC_OUT_CONVEX, 0.75, 0.25, dt, nullptr, from, stream)))
-    return st;
-  if (fill && (st = swc_halo_fill(grid, scheme->dtype, 5, w2, bcs, 0, stream)))
-    return st;
-  return plain_stage(grid, scheme, (const void* const*)w2, cu, u,
-                     SWC_OUT_CONVEX, 1.0 / 3.0, 2.0 / 3.0, dt, dtmin, from,
-                     stream);
+  void* const* in[3] = {u, w1, w2};
+  for (int k = 0; k < order; ++k) {
+    if (k > 0 && fill &&
+        (st = swc_halo_fill(grid, scheme->dtype, 5, in[k], bcs, 0, stream)))
+      return st;
+    if ((st = plain_launch(scheme, a[k], stream))) return st;
+  }
+  return SWC_OK;
 }
 
 // Where the first stage of a functional call may read the caller's fields as

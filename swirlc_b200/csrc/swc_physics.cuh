@@ -78,7 +78,7 @@ __device__ __forceinline__ double rcp_normal(double a) {
 // w_0 = (b_1 b_2 s)^2 and so on. The power of two s brings the largest product
 // to [1, 2), so that no weight that counts leaves the normal range, however
 // large or small the b_r. b_r above 2^511, whose squares overflow, count as
-// 2^511. Two steps of KH 112^3: 1238 us; with one reciprocal per b_r 1281;
+// 2^511. A step of KH 112^3: 1238 us; with one reciprocal per b_r 1281;
 // with a fixed scale, whose products leave the normal range for fields below
 // 1e-8 and above 1e62, 1193.
 __device__ __forceinline__ double limit_511(double b) {
