@@ -117,26 +117,27 @@ __global__ void halo_clear_kernel(const ShellArgs a, int total) {
 // launch reads and writes each field once; a copy per field, the fill and a
 // memset per right-hand side were twelve launches, and their host time was
 // most of a small call (a right-hand side at 61 x 47 x 33: 101 us).
-template <typename T, int NF>
+template <typename T, int NF, bool PLAIN>
 __global__ void __launch_bounds__(kCopyY* kCopyX)
     halo_copy_kernel(const ShellArgs a, const ShellCopy c) {
   const int cy = blockIdx.x * kCopyY + threadIdx.x;
-  const int cx = blockIdx.y * kCopyX * kCopyRows + threadIdx.y;
-  if (cy < a.ny + 2 * a.h) halo_copy_elem<T, NF>(a, c, cx, cy, blockIdx.z);
+  const int cx = c.x0 + blockIdx.y * kCopyX * kCopyRows + threadIdx.y;
+  if (cy < a.ny + 2 * a.h)
+    halo_copy_elem<T, NF, PLAIN>(a, c, cx, cy, c.z0 + blockIdx.z);
 }
-template <typename T>
+template <typename T, bool PLAIN>
 void launch_halo_copy(const ShellArgs& a, const ShellCopy& c, dim3 blocks,
                       cudaStream_t s) {
   const dim3 t(kCopyY, kCopyX);
   switch (a.nf) {
-    case 1: halo_copy_kernel<T, 1><<<blocks, t, 0, s>>>(a, c); break;
-    case 2: halo_copy_kernel<T, 2><<<blocks, t, 0, s>>>(a, c); break;
-    case 3: halo_copy_kernel<T, 3><<<blocks, t, 0, s>>>(a, c); break;
-    case 4: halo_copy_kernel<T, 4><<<blocks, t, 0, s>>>(a, c); break;
-    case 5: halo_copy_kernel<T, 5><<<blocks, t, 0, s>>>(a, c); break;
-    case 6: halo_copy_kernel<T, 6><<<blocks, t, 0, s>>>(a, c); break;
-    case 7: halo_copy_kernel<T, 7><<<blocks, t, 0, s>>>(a, c); break;
-    default: halo_copy_kernel<T, 8><<<blocks, t, 0, s>>>(a, c); break;
+    case 1: halo_copy_kernel<T, 1, PLAIN><<<blocks, t, 0, s>>>(a, c); break;
+    case 2: halo_copy_kernel<T, 2, PLAIN><<<blocks, t, 0, s>>>(a, c); break;
+    case 3: halo_copy_kernel<T, 3, PLAIN><<<blocks, t, 0, s>>>(a, c); break;
+    case 4: halo_copy_kernel<T, 4, PLAIN><<<blocks, t, 0, s>>>(a, c); break;
+    case 5: halo_copy_kernel<T, 5, PLAIN><<<blocks, t, 0, s>>>(a, c); break;
+    case 6: halo_copy_kernel<T, 6, PLAIN><<<blocks, t, 0, s>>>(a, c); break;
+    case 7: halo_copy_kernel<T, 7, PLAIN><<<blocks, t, 0, s>>>(a, c); break;
+    default: halo_copy_kernel<T, 8, PLAIN><<<blocks, t, 0, s>>>(a, c); break;
   }
 }
 
@@ -773,34 +774,46 @@ int swc_halo_copy(const SwcGrid* grid, int32_t dtype, int32_t nfields,
   const long long nxa = grid->nx + 2LL * h, nya = grid->ny + 2LL * h,
                   nza = grid->nz + 2LL * h;
   ShellArgs sa;
-  const int rows = kCopyX * kCopyRows;
-  const long long by = (nxa + rows - 1) / rows;
-  if (by <= 65535 && nza <= 65535 &&
-      shell_args(grid, nfields, src, bcs, any_prim, sa)) {
-    ShellCopy c;
-    memset(&c, 0, sizeof(c));
-    for (int i = 0; i < nfields; ++i) {
-      c.dst[i] = dst[i];
-      c.clear[i] = clear ? clear[i] : nullptr;
-    }
-    const dim3 blocks((unsigned)((nya + kCopyY - 1) / kCopyY), (unsigned)by,
-                      (unsigned)nza);
-    if (dtype == SWC_F32) launch_halo_copy<float>(sa, c, blocks, s);
-    else launch_halo_copy<double>(sa, c, blocks, s);
-    note_launch();
-    return check_launch("halo_copy");
-  }
-  // Conditions on primitives, unfilled sides, periodic dims narrower than the
-  // halo: copies, then the fill's passes.
-  const size_t bytes = (size_t)(grid->sz * nza) * (dtype == SWC_F32 ? 4 : 8);
+  ShellCopy c;
+  memset(&c, 0, sizeof(c));
   for (int i = 0; i < nfields; ++i) {
-    cudaError_t e = cudaMemcpyAsync(dst[i], src[i], bytes,
-                                    cudaMemcpyDeviceToDevice, s);
-    if (e == cudaSuccess && clear) e = cudaMemsetAsync(clear[i], 0, bytes, s);
-    if (e != cudaSuccess)
-      return fail(SWC_ERR_LAUNCH, "halo copy: %s", cudaGetErrorString(e));
+    c.dst[i] = dst[i];
+    c.clear[i] = clear ? clear[i] : nullptr;
   }
-  return swc_halo_fill(grid, dtype, nfields, dst, bcs, rho_index, stream);
+  const bool plain = !shell_args(grid, nfields, src, bcs, any_prim, sa);
+  if (plain) {
+    // Conditions on primitives, unfilled sides, periodic dims narrower than
+    // the halo: plain copies, then the fill's passes. The copies are the same
+    // kernel's: the cells between the rows and planes of a grid with wider
+    // strides are somebody else's.
+    memset(&sa, 0, sizeof(sa));
+    sa.nf = nfields;
+    for (int i = 0; i < nfields; ++i) sa.fld[i].f = const_cast<void*>(src[i]);
+    sa.nx = grid->nx; sa.ny = grid->ny; sa.nz = grid->nz; sa.h = h;
+    sa.sx = grid->sx; sa.sz = grid->sz;
+  }
+  // At most 65535 blocks along y and z of a launch.
+  const long long most = 65535, rows = kCopyX * kCopyRows;
+  for (long long z = 0; z < nza; z += most)
+    for (long long x = 0; x < nxa; x += most * rows) {
+      c.z0 = (int)z;
+      c.x0 = (int)x;
+      const dim3 blocks(
+          (unsigned)((nya + kCopyY - 1) / kCopyY),
+          (unsigned)std::min(most, (nxa - x + rows - 1) / rows),
+          (unsigned)std::min(most, nza - z));
+      if (dtype == SWC_F32)
+        plain ? launch_halo_copy<float, true>(sa, c, blocks, s)
+              : launch_halo_copy<float, false>(sa, c, blocks, s);
+      else
+        plain ? launch_halo_copy<double, true>(sa, c, blocks, s)
+              : launch_halo_copy<double, false>(sa, c, blocks, s);
+      note_launch();
+      if ((st = check_launch("halo_copy"))) return st;
+    }
+  return plain ? swc_halo_fill(grid, dtype, nfields, dst, bcs, rho_index,
+                               stream)
+               : SWC_OK;
 }
 
 // Checks and the kernel arguments shared by swc_rk_stage and

@@ -373,11 +373,13 @@ __device__ __forceinline__ void halo_shell_bc_elem(const ShellArgs& a, int t) {
 
 // Copies with filled halos: dst[f] of every padded cell takes what
 // halo_shell_bc_elem would leave in a copy of the field, which stays as it
-// is; `clear` (where not NULL, for all fields or none) gets zeros in its halo
-// cells, as a right-hand side returns them.
+// is, or (PLAIN) the field's own value; `clear` (where not NULL, for all
+// fields or none) gets zeros in its halo cells, as a right-hand side returns
+// them. A launch covers the cells from (x0, z0) on.
 struct ShellCopy {
   void* dst[SWC_MAX_FIELDS];
   void* clear[SWC_MAX_FIELDS];
+  int x0, z0;
 };
 // A block of 32 x 8 threads takes 32 cells along y by 16 rows, two per thread.
 constexpr int kCopyY = 32, kCopyX = 8, kCopyRows = 2;
@@ -385,7 +387,7 @@ constexpr int kCopyY = 32, kCopyX = 8, kCopyRows = 2;
 // The cells (cx + k * kCopyX, cy, cz), k < kCopyRows, of the padded grid. The
 // loads of all cells with one source for every field come before any store,
 // so that they are in flight together.
-template <typename T, int NF>
+template <typename T, int NF, bool PLAIN>
 __device__ __forceinline__ void halo_copy_elem(const ShellArgs& a,
                                                const ShellCopy& c, int cx,
                                                int cy, int cz) {
@@ -397,7 +399,12 @@ __device__ __forceinline__ void halo_copy_elem(const ShellArgs& a,
   for (int k = 0; k < kCopyRows; ++k) {
     const int x = cx + k * kCopyX;
     long long os;
-    same[k] = x < nxa && shell_source(a, x, cy, cz, os);
+    if constexpr (PLAIN) {
+      os = cz * a.sz + x * a.sx + cy;
+      same[k] = x < nxa;
+    } else {
+      same[k] = x < nxa && shell_source(a, x, cy, cz, os);
+    }
 #pragma unroll
     for (int f = 0; f < NF; ++f)
       if (same[k]) v[k][f] = static_cast<const T*>(a.fld[f].f)[os];
