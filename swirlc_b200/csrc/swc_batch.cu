@@ -439,17 +439,23 @@ extern "C" int swc_batch_step(const SwcScheme* sc, int32_t order,
     const int rc = check_member(members[i], i, need);
     if (rc) return rc;
   }
-  // Tiles: 16x16 unless the member asks for 8x32 (which suits members at
-  // most 8 cells wide in y, and is not offered for f64 WENO5, whose layout
-  // fills the whole of shared memory). The 16x16 instance reproduces swc_rk_step bit for bit; the
-  // 8x32 instance of the same arithmetic is scheduled differently by the
-  // compiler and can differ from it in the last bit.
-  const bool narrow_ok = (sc->dtype == SWC_F32 || sc->interp != SWC_WENO5) &&
-                         batch_smem(sc, 2) <= kSmemLimit;
+  // Tiles: 16x16 unless the member asks for 8x32, which suits members at most
+  // 8 cells wide in y. Double-precision WENO5 has no 8x32 tile: its layout
+  // (222,912 bytes) would fit since the planes are converted in place, but
+  // that instance has never been run or timed, and a double-precision CTA has
+  // its SM to itself with either tile. The 16x16 instance reproduces
+  // swc_rk_step bit for bit; the 8x32 instance of the same arithmetic is
+  // scheduled differently by the compiler and can differ from it in the last
+  // bit.
+  const bool narrow_none = sc->dtype == SWC_F64 && sc->interp == SWC_WENO5;
   std::vector<Plan> plans(nmembers);
   for (int i = 0; i < nmembers; ++i) {
     plans[i].m = &members[i];
-    if (members[i].tile == 2 && !narrow_ok)
+    if (members[i].tile == 2 && narrow_none)
+      return record_error(SWC_ERR_UNSUPPORTED,
+                          "member %d: tile 8x32 is not available for "
+                          "double-precision WENO5", i);
+    if (members[i].tile == 2 && batch_smem(sc, 2) > kSmemLimit)
       return record_error(SWC_ERR_UNSUPPORTED,
                           "member %d: tile 8x32 needs %zu bytes of shared "
                           "memory for this scheme and dtype", i,
