@@ -64,10 +64,11 @@ __device__ __forceinline__ double cfl_limit_or_flag(T rho, T p, T rhoe, T l) {
 }
 
 // 1/a of a normal, finite a whose reciprocal is normal too: the hardware's
-// starting value x (relative error below 2^-19) and one Householder step of
-// third order, x (1 + r + r^2) with r = 1 - a x, whose remainder r^3 is below
-// 2^-57. About half the instructions of the correctly rounded quotient and no
-// branch; the result is within one unit in the last place of it.
+// starting value x (relative error below 2^-19) and one step of Householder's
+// third-order iteration, x (1 + r + r^2) with r = 1 - a x, whose remainder r^3
+// is below 2^-57. About half the instructions of the correctly rounded quotient
+// and no branch; the result is within one unit in the last place of it (tested
+// over every exponent).
 __device__ __forceinline__ double rcp_normal(double a) {
   double x;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(a));

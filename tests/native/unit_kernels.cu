@@ -27,7 +27,18 @@ __global__ void weno5_vjp_kernel(int n, const T* v, const T* rb, const T* lb,
   }
 }
 
+__global__ void rcp_normal_kernel(int n, const double* a, double* out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) out[i] = swc::rcp_normal(a[i]);
+}
+
 }  // namespace
+
+extern "C" int unit_rcp_normal(int n, const void* a, void* out) {
+  rcp_normal_kernel<<<(n + 127) / 128, 128>>>(
+      n, static_cast<const double*>(a), static_cast<double*>(out));
+  return cudaGetLastError() != cudaSuccess;
+}
 
 extern "C" int unit_weno5_vjp(int n, int f64, const void* v, const void* rb,
                               const void* lb, void* vb) {

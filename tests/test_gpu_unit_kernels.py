@@ -51,3 +51,28 @@ def test_weno5_reverse_beside_a_jump(lib, dtype, low, ratio, noise):
   for k in range(5):
     worst = (np.abs(got[k] - want[k]) / (1000 * u * size[k])).max()
     assert worst <= 1, f'cell {k}: {float(worst):.3g} of the bound'
+
+
+def test_rcp_normal_within_one_unit(lib):
+  """The reciprocal of the WENO denominators in double precision is within one
+  unit in the last place of 1 / a wherever a and 1 / a are normal: random
+  mantissas over all exponents, values next to powers of two, and the range of
+  the denominators (weights up to 4, factors 2 to 12)."""
+  rng = np.random.default_rng(3)
+  n = 400000
+  a = np.ldexp(rng.uniform(1, 2, n), rng.integers(-1022, 1022, n))
+  powers = np.ldexp(1.0, np.arange(-1021, 1022))
+  near = np.concatenate([powers + j * np.spacing(powers) for j in range(4)] +
+                        [powers - j * np.spacing(powers) / 2
+                         for j in range(1, 4)])
+  ends = np.array([np.finfo(np.float64).tiny, 2.0**1022])
+  a = np.concatenate([a, near, ends, rng.uniform(1, 80, n)])
+  a *= np.where(rng.integers(0, 2, a.size) == 1, 1.0, -1.0)
+  da = torch.tensor(a, device='cuda')
+  out = torch.empty_like(da)
+  torch.cuda.synchronize()
+  assert lib.unit_rcp_normal(a.size, _ptr(da), _ptr(out)) == 0
+  torch.cuda.synchronize()
+  want = 1.0 / a
+  off = np.abs(out.cpu().numpy().view(np.int64) - want.view(np.int64))
+  assert off.max() <= 1, (off.max(), a[off.argmax()])
