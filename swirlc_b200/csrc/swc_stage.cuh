@@ -23,8 +23,6 @@
 // register pair. Everything up to the stage update is explicitly rounded.
 #pragma once
 
-#include <math.h>
-
 #include <type_traits>
 
 #include "swc_physics.cuh"
@@ -43,13 +41,11 @@ struct StageArgs {
   const void* u0[SWC_MAX_FIELDS];
   void* uout[SWC_MAX_FIELDS];
   int mode;
-  // Combination w0 u0 + w1 (uk + dt L) of the caller's weights
-  // (stage_weights): SWC_OUT_CONVEX forms c0 u0 + c1 ((uk - u0) + dt L) with
-  // c0 = w0 + w1, where the change is rounded at its own size and the result
-  // once, and 1/3 and 2/3 rounded to 32 bits, which add up to 1 + 3e-8, do not
-  // scale the state (the error of a gradient with respect to the fields
-  // against 64 bits fell from 4.5e-6 to 2.3e-6); kOutWeighted forms
-  // c1 ((uk + c0 u0) + dt L) with c0 = w0 / w1.
+  // SWC_OUT_CONVEX forms c0 u0 + c1 ((uk - u0) + dt L): for the caller's
+  // w0 u0 + w1 (uk + dt L) c0 is w0 + w1 (stage_weights). The change is rounded
+  // at its own size and the result once, and 1/3 and 2/3 rounded to 32 bits,
+  // which add up to 1 + 3e-8, do not scale the state: the error of a gradient
+  // with respect to the fields against 64 bits fell from 4.5e-6 to 2.3e-6.
   double c0, c1;
   const double* dt;
   double* dtmin_out;
@@ -66,25 +62,13 @@ struct StageArgs {
   int halo_from[3];
 };
 enum { kHaloStored, kHaloWrapped, kHaloClamped };
-enum { kOutWeighted = SWC_OUT_AVERAGE + 1 };
 // mode, c0 and c1 of a stage of the caller's mode and weights; the average
-// w0 (u0 + uk + dt L) is the combination with both weights w0. The change is
-// taken where |w1| <= 2 |w0|, as in every Runge-Kutta stage: there the w1 u0
-// taken out and put back is no larger than twice the u0 term itself. Elsewhere
-// (w0 = 0, say, with a u0 that has nothing to do with uk) it could drown the
-// result.
+// w0 (u0 + uk + dt L) is the combination with both weights w0.
 inline void stage_weights(StageArgs& a, int mode, double w0, double w1) {
-  if (mode == SWC_OUT_AVERAGE) {
-    mode = SWC_OUT_CONVEX;
-    w1 = w0;
-  }
-  a.mode = mode;
-  a.c0 = w0 + w1;
-  a.c1 = w1;
-  if (mode == SWC_OUT_CONVEX && !(fabs(w1) <= 2.0 * fabs(w0))) {
-    a.mode = kOutWeighted;
-    a.c0 = w0 / w1;
-  }
+  const double second = mode == SWC_OUT_AVERAGE ? w0 : w1;
+  a.mode = mode == SWC_OUT_AVERAGE ? SWC_OUT_CONVEX : mode;
+  a.c0 = w0 + second;
+  a.c1 = second;
 }
 
 // Padded coordinate a halo cell c of a dim of n cells is read from.
@@ -767,12 +751,6 @@ __device__ __forceinline__ void stage_body(const StageArgs& a,
         u0c[v] = a.mode == SWC_OUT_CONVEX
                      ? __ldg(static_cast<const T*>(a.u0[v]) + o)
                      : T(0);
-      }
-      if (a.mode == kOutWeighted) {
-#pragma unroll
-        for (int v = 0; v < NF; ++v)
-          ukc[v] = O1::fma(T(a.c0), __ldg(static_cast<const T*>(a.u0[v]) + o),
-                           ukc[v]);
       }
     }
     if (zc + 1 < z1) {
