@@ -142,6 +142,8 @@ struct One<float> {
   static __device__ __forceinline__ V rcpn(V a) { return 1.0f / a; }
   // a / b as a times the reciprocal of b (what the fast-math quotient is).
   static __device__ __forceinline__ V div(V a, V b) { return __fmul_rn(a, 1.0f / b); }
+  // a / b with rb = rcp(b) at hand.
+  static __device__ __forceinline__ V quot(V a, V, V rb) { return __fmul_rn(a, rb); }
   // x where p > 0, else 0.
   static __device__ __forceinline__ V sel_pos(V p, V x) { return p > 0.0f ? x : 0.0f; }
   template <class F>
@@ -159,6 +161,12 @@ struct One<double> {
   static __device__ __forceinline__ V rcp(V a) { return 1.0 / a; }
   static __device__ __forceinline__ V rcpn(V a) { return rcp_normal(a); }
   static __device__ __forceinline__ V div(V a, V b) { return __ddiv_rn(a, b); }
+  // The product a rb is off by up to 2 units of roundoff; its remainder, exact
+  // in an FMA, leaves one.
+  static __device__ __forceinline__ V quot(V a, V b, V rb) {
+    const V q = __dmul_rn(a, rb);
+    return __fma_rn(__fma_rn(-q, b, a), rb, q);
+  }
   static __device__ __forceinline__ V sel_pos(V p, V x) { return p > 0.0 ? x : 0.0; }
   template <class F>
   static __device__ __forceinline__ V map3(F f, V a, V b, V c) { return f(a, b, c); }
@@ -736,7 +744,9 @@ __device__ __forceinline__ void viscous_flux(T ra, T rb, const T* ua,
   const T tau[3] = {O::mul(mu2, O::fma(T(-1.0 / 3.0), div, bd[0])),
                     O::mul(mu, O::add(bd[1], g10)),
                     O::mul(mu, O::add(bd[2], g20))};
-  const T dt = O::sub(O::mul(pb, O::rcp(rb)), O::mul(pa, O::rcp(ra)));
+  // Temperatures (times R) differ little from cell to cell: what their
+  // quotients are off by is most of the heat flux's error.
+  const T dt = O::sub(O::quot(pb, rb, O::rcp(rb)), O::quot(pa, ra, O::rcp(ra)));
   const T q = O::mul(O::mul(O::mul(kq, mu2), dt), rh);  // -q_0
   const T d2 = O::fma(
       O::add(ua[2], ub[2]), tau[2],
