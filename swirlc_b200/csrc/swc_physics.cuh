@@ -142,8 +142,12 @@ struct One<float> {
   static __device__ __forceinline__ V rcpn(V a) { return 1.0f / a; }
   // a / b as a times the reciprocal of b (what the fast-math quotient is).
   static __device__ __forceinline__ V div(V a, V b) { return __fmul_rn(a, 1.0f / b); }
-  // a / b with rb = rcp(b) at hand.
-  static __device__ __forceinline__ V quot(V a, V, V rb) { return __fmul_rn(a, rb); }
+  // a / b with rb = rcp(b) at hand: the product a rb is off by 2 units of
+  // roundoff and more; its remainder, exact in an FMA, leaves one.
+  static __device__ __forceinline__ V quot(V a, V b, V rb) {
+    const V q = __fmul_rn(a, rb);
+    return __fmaf_rn(__fmaf_rn(-q, b, a), rb, q);
+  }
   // x where p > 0, else 0.
   static __device__ __forceinline__ V sel_pos(V p, V x) { return p > 0.0f ? x : 0.0f; }
   template <class F>
@@ -161,8 +165,6 @@ struct One<double> {
   static __device__ __forceinline__ V rcp(V a) { return 1.0 / a; }
   static __device__ __forceinline__ V rcpn(V a) { return rcp_normal(a); }
   static __device__ __forceinline__ V div(V a, V b) { return __ddiv_rn(a, b); }
-  // The product a rb is off by up to 2 units of roundoff; its remainder, exact
-  // in an FMA, leaves one.
   static __device__ __forceinline__ V quot(V a, V b, V rb) {
     const V q = __dmul_rn(a, rb);
     return __fma_rn(__fma_rn(-q, b, a), rb, q);
