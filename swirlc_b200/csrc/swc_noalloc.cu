@@ -17,9 +17,10 @@
 // it and is shared by all calls, so calls that overlap on the GPU (other
 // streams, other host threads on the same device) race on it. Nothing in it
 // has to start at zero: the step writes each work state's interior before
-// reading it, and the halo fill writes its halos, as with caller buffers
-// (except on sides set to SWC_BC_NONE, whose halos keep old contents there
-// exactly as they would in a reused caller buffer).
+// reading it, and its halos are filled, or not read at all where a stage takes
+// them from the interior, as with caller buffers (except on sides set to
+// SWC_BC_NONE, whose halos keep old contents there exactly as they would in a
+// reused caller buffer).
 #include <cuda_runtime.h>
 #include <stdint.h>
 
